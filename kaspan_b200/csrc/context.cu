@@ -220,8 +220,10 @@ struct phase_clock
 };
 
 // The whole path on a resident graph; writes the canonical ids into scc_id.
+// own_transpose: (bh, bc) was built here from the CSR, so checking the CSR
+// checks it too (a transpose of valid rows is valid).
 void
-run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options const& opt, kspn_stats* st)
+run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options const& opt, kspn_stats* st, bool own_transpose = false)
 {
   auto& ws = ctx->ws;
   ensure_workspace(ctx, g.n, g.m);
@@ -245,7 +247,14 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
   KSPN_CUDA(cudaEventRecord(t_begin, ctx->stream));
   phase_clock clk{ ctx, st };
   clk.start();
-  if (opt.validate) validate(ctx, g);
+  // the resident pipeline queues the checks ahead of its launches, which
+  // leave the graph's rows alone when a fault bit is set, and reads the bits
+  // with its results: no host round trip of their own
+  bool const resident = opt.pipeline == KSPN_PIPELINE_FAST && g.n != 0 && !ctx->prof && resident_fits(g);
+  if (opt.validate) {
+    if (resident) validate_async(ctx, g, !own_transpose);
+    else validate(ctx, g, !own_transpose);
+  }
   if (g.n == 0) return;
 
   uint32_t* und         = ws.und;
@@ -359,7 +368,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
         if ((decided - d0) * 64 < left) break;
       }
     };
-    if (!ctx->prof && resident_fits(g)) {
+    if (resident) {
       // trim_1_first, then FW-BW and the trim fixpoint in ONE persistent
       // launch that takes the pivot from device memory: one host sync
       trim_1_first_async(ctx, g, und);
@@ -370,6 +379,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
       KSPN_CUDA(cudaMemcpyAsync(ctx->h_ctr, ws.ctr, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
       KSPN_CUDA(cudaEventRecord(ctx->ev[3], ctx->stream));
       KSPN_CUDA(cudaEventSynchronize(ctx->ev[3]));
+      if (opt.validate) validate_check(ctx->h_ctr[CTR_ERR]);
       resident_result r = fw_bw_trim_result(ctx, g, opt, st);
       if (r.resumed) {
         // the phase clock's end after the resume launch
@@ -818,7 +828,7 @@ kspn_scc_device(kspn_context* ctx, uint32_t n, uint64_t m, const uint64_t* d_fw_
     bind_device(ctx);
     graph_store  store;
     dgraph const g = with_transpose(ctx, n, m, d_fw_head, d_fw_csr, d_bw_head, d_bw_csr, store);
-    run_pipeline(ctx, g, d_scc_id, o, stats);
+    run_pipeline(ctx, g, d_scc_id, o, stats, d_bw_head == nullptr);
   });
 }
 
@@ -859,7 +869,7 @@ kspn_scc(kspn_context* ctx, uint32_t n, uint64_t m, const uint64_t* fw_head, con
       upload_transpose(ctx, n, m, fw_head, fw_csr, dfh, dfc, dbh, dbc, 0);
     }
     dgraph const g{ n, m, dfh, dfc, dbh, dbc };
-    run_pipeline(ctx, g, dout, o, stats);
+    run_pipeline(ctx, g, dout, o, stats, !has_bw);
     if (n) KSPN_CUDA(cudaMemcpyAsync(scc_id, dout, static_cast<size_t>(n) * 4, cudaMemcpyDeviceToHost, s));
     KSPN_CUDA(cudaStreamSynchronize(s));
   });

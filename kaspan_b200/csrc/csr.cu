@@ -80,15 +80,55 @@ k_compact_edges(uint64_t m_raw, uint32_t const* __restrict__ s, uint32_t const* 
   }
 }
 
-__global__ void
-k_validate(uint32_t n, uint64_t m, uint64_t const* __restrict__ head, uint32_t const* __restrict__ csr, uint32_t* __restrict__ err)
+// One direction's checks per grid row (blockIdx.y: CSR, transpose), both in
+// one launch.  A pure stream: 8(n+1) + 4m bytes per direction, so the ids
+// are read 16 bytes at a time with VA_ILP loads in flight per thread (the
+// rows' array may start at any 4-byte address: the ids before the first and
+// after the last 16-byte boundary are read one by one).  R-MAT scale 24
+// (n 16.8 M, m 263 M), per direction: 443 us with one 4-byte load per
+// thread and step, 245 us this way.
+constexpr int VA_THREADS = 256, VA_ILP = 4;
+struct graph_rows
 {
-  uint64_t const stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
-    if (head[i] > head[i + 1]) atomicOr(err, 1u);
-  if (blockIdx.x == 0 && threadIdx.x == 0 && (head[0] != 0 || head[n] != m)) atomicOr(err, 2u);
-  for (uint64_t e = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += stride)
-    if (csr[e] >= n) atomicOr(err, 4u);
+  uint64_t const* head;
+  uint32_t const* csr;
+};
+
+__global__ void __launch_bounds__(VA_THREADS)
+k_validate(uint32_t n, uint64_t m, graph_rows fw, graph_rows bw, uint32_t* __restrict__ err)
+{
+  graph_rows const g      = blockIdx.y ? bw : fw;
+  uint64_t const   stride = static_cast<uint64_t>(gridDim.x) * VA_THREADS;
+  uint64_t const   tid    = static_cast<uint64_t>(blockIdx.x) * VA_THREADS + threadIdx.x;
+  uint32_t         bad    = 0;
+  for (uint64_t i0 = tid; i0 < n; i0 += VA_ILP * stride) {
+    uint64_t a[VA_ILP], b[VA_ILP];
+#pragma unroll
+    for (int k = 0; k < VA_ILP; ++k) {
+      uint64_t const i = i0 + k * stride;
+      a[k] = b[k] = 0;
+      if (i < n) a[k] = g.head[i], b[k] = g.head[i + 1];
+    }
+#pragma unroll
+    for (int k = 0; k < VA_ILP; ++k) bad |= a[k] > b[k] ? 1u : 0u;
+  }
+  if (tid == 0 && (g.head[0] != 0 || g.head[n] != m)) bad |= 2u;
+  uint64_t const lead = min(m, ((16u - (reinterpret_cast<uintptr_t>(g.csr) & 15u)) & 15u) / 4u);
+  uint64_t const nv   = (m - lead) / 4;
+  auto const*    v    = reinterpret_cast<uint4 const*>(g.csr + lead);
+  uint32_t       most = 0; // largest id seen
+  for (uint64_t i0 = tid; i0 < nv; i0 += VA_ILP * stride) {
+    uint4 x[VA_ILP];
+#pragma unroll
+    for (int k = 0; k < VA_ILP; ++k) x[k] = i0 + k * stride < nv ? v[i0 + k * stride] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int k = 0; k < VA_ILP; ++k) most = max(most, max(max(x[k].x, x[k].y), max(x[k].z, x[k].w)));
+  }
+  uint64_t const rest = m - lead - nv * 4; // at most 3 ids past the last boundary
+  if (tid < lead) most = max(most, g.csr[tid]);
+  if (tid < rest) most = max(most, g.csr[lead + nv * 4 + tid]);
+  if (m && most >= n) bad |= 4u;
+  if (bad) atomicOr(err, bad);
 }
 
 // src[e - e0] = u for the edges e in [e0, e1) of rows [u_lo, u_hi) (rows
@@ -471,25 +511,33 @@ build_csr(kspn_context* ctx, uint32_t n, uint64_t m_raw, uint32_t* src, uint32_t
 }
 
 void
-validate(kspn_context* ctx, dgraph const& g)
+validate_async(kspn_context* ctx, dgraph const& g, bool transpose_too)
 {
-  cudaStream_t const s = ctx->stream;
-  uint32_t*          err = ctx->ws.ctr + CTR_ERR;
-  KSPN_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), s));
-  uint64_t const items = g.m > g.n ? g.m : g.n;
-  k_validate<<<grid_for(items, 256), 256, 0, s>>>(g.n, g.m, g.fh, g.fc, err);
-  if (g.bh != g.fh) k_validate<<<grid_for(items, 256), 256, 0, s>>>(g.n, g.m, g.bh, g.bc, err);
+  uint64_t const items = std::max<uint64_t>(g.m / (4 * VA_ILP), g.n / VA_ILP) + 1;
+  unsigned const gx    = static_cast<unsigned>(std::min<uint64_t>(div_up(items, VA_THREADS), 148ull * 4)); // both directions resident at once
+  k_validate<<<dim3(gx, transpose_too && g.bh != g.fh ? 2 : 1), VA_THREADS, 0, ctx->stream>>>(g.n, g.m, graph_rows{ g.fh, g.fc }, graph_rows{ g.bh, g.bc }, ctx->ws.ctr + CTR_ERR);
   KSPN_CHECK_LAUNCH();
-  ctx->launches += 2;
+  ctx->launches += 1;
+}
+
+void
+validate_check(uint32_t e)
+{
+  if (!e) return;
+  std::string what = "invalid graph:";
+  if (e & 1u) what += " offsets decrease;";
+  if (e & 2u) what += " head[0] != 0 or head[n] != m;";
+  if (e & 4u) what += " neighbour id >= n;";
+  throw error{ KSPN_ERR_INVALID_GRAPH, what };
+}
+
+void
+validate(kspn_context* ctx, dgraph const& g, bool transpose_too)
+{
+  KSPN_CUDA(cudaMemsetAsync(ctx->ws.ctr + CTR_ERR, 0, sizeof(uint32_t), ctx->stream));
+  validate_async(ctx, g, transpose_too);
   read_counters(ctx);
-  uint32_t const e = ctx->h_ctr[CTR_ERR];
-  if (e) {
-    std::string what = "invalid graph:";
-    if (e & 1u) what += " offsets decrease;";
-    if (e & 2u) what += " head[0] != 0 or head[n] != m;";
-    if (e & 4u) what += " neighbour id >= n;";
-    throw error{ KSPN_ERR_INVALID_GRAPH, what };
-  }
+  validate_check(ctx->h_ctr[CTR_ERR]);
 }
 
 } // namespace kspn

@@ -556,7 +556,14 @@ void     transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* fh
 constexpr uint64_t UPLOAD_CHUNK = 8ull << 20;
 void     upload_transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* h_fh, uint32_t const* h_fc, uint64_t* dfh, uint32_t* dfc, uint64_t* dbh, uint32_t* dbc, uint64_t chunk);
 uint64_t build_csr(kspn_context* ctx, uint32_t n, uint64_t m_raw, uint32_t* src, uint32_t* dst, uint64_t* head, uint32_t* csr);
-void     validate(kspn_context* ctx, dgraph const& g);
+// Input checks.  validate: launches the checks, waits and throws
+// KSPN_ERR_INVALID_GRAPH.  validate_async only launches them: the fault bits
+// are in ws.ctr[CTR_ERR] (zeroed by the caller), for validate_check once the
+// host has read them.  transpose_too: false when the transpose was built
+// here from the checked CSR.
+void     validate(kspn_context* ctx, dgraph const& g, bool transpose_too = true);
+void     validate_async(kspn_context* ctx, dgraph const& g, bool transpose_too);
+void     validate_check(uint32_t e);
 
 // gen.cu
 void gen_gnm(kspn_context* ctx, uint32_t n, uint64_t draws, uint64_t seed, uint32_t* src, uint32_t* dst);

@@ -799,6 +799,7 @@ struct fwbw_args
   uint32_t           drop_barrier; // test hook: the last block leaves this barrier of the launch (0 = off)
   uint64_t           aw_exact;     // worklist items after which warps take their finds exactly
   float const*       model;        // pivot MLP parameters: the launch scores its pivot first (null: no check)
+  uint32_t const*    gate;         // not null and *gate != 0: the input check failed, the launch does nothing
   void*              jsave;        // the level loop's saved control (handoff, resume)
   uint32_t           resume;       // 1: continue a launch that handed off, at its worklist phase
 };
@@ -2132,6 +2133,7 @@ __global__ void __launch_bounds__(R_THREADS, MINB)
 k_fwbw(fwbw_args a)
 {
   __shared__ fwbw_smem sm;
+  if (a.gate && __ldcg(a.gate)) return; // the same word for every block
   reach_state* const   st    = a.st;
   unsigned long long   epoch = __ldcg(&a.bar->epoch);
   uint32_t const       words = (a.n + 31) / 32;
@@ -2512,7 +2514,7 @@ namespace {
 // caller synchronises, then calls check_persistent.
 void
 launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t pivot, bool trim, kspn_options const& opt, kspn_stats* st, bool min_ids,
-                  cudaEvent_t after_kernel = nullptr, bool ids_at_end = true, float const* model = nullptr)
+                  cudaEvent_t after_kernel = nullptr, bool ids_at_end = true, float const* model = nullptr, bool gated = false)
 {
   auto&       ws   = ctx->ws;
   auto* const rs   = reinterpret_cast<reach_state*>(ws.rstate);
@@ -2569,6 +2571,7 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
   // an earlier switch only cuts duplicates; a later one could overrun the worklist's bound
   a.aw_exact     = opt.aw_exact_after && opt.aw_exact_after < ws.aw_entries / 2 ? opt.aw_exact_after : ws.aw_entries / 2;
   a.model        = model;
+  a.gate         = gated ? ws.ctr + CTR_ERR : nullptr;
   a.jsave        = static_cast<char*>(ws.gbar) + 2048;
   a.resume       = 0;
   static_assert(sizeof(fwbw_args) <= sizeof(ctx->fwbw_last), "launch arguments must fit their copy in the context");
@@ -2659,7 +2662,7 @@ fw_bw_trim_async(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* sc
 {
   // with the learned rule the launch scores trim_1_first's pivot itself
   float const* model = opt.learned_pivot && ctx->pivot_model ? ctx->pivot_model : nullptr;
-  launch_persistent(ctx, g, und, scc_id, static_cast<uint32_t>(PIVOT_FROM_DEVICE), true, opt, st, true, after_kernel, true, model);
+  launch_persistent(ctx, g, und, scc_id, static_cast<uint32_t>(PIVOT_FROM_DEVICE), true, opt, st, true, after_kernel, true, model, opt.validate != 0);
 }
 
 resident_result
