@@ -757,7 +757,6 @@ struct batch_plan
   uint32_t* words = nullptr;
   uint64_t* word_off = nullptr;
   uint32_t* hist = nullptr;
-  uint32_t* part = nullptr;
   uint64_t* part64 = nullptr;
   uint32_t* und = nullptr;
   uint32_t* vis_a = nullptr;
@@ -822,7 +821,6 @@ carve_plan(batch_plan& p, char* base, uint32_t G, uint64_t N, size_t* bytes_out)
   p.words    = reinterpret_cast<uint32_t*>(take(4 * (G + 1)));
   p.word_off = reinterpret_cast<uint64_t*>(take(8 * (G + 1)));
   p.hist     = reinterpret_cast<uint32_t*>(take(4 * hist_n));
-  p.part     = reinterpret_cast<uint32_t*>(take(4 * part_n));
   p.part64   = reinterpret_cast<uint64_t*>(take(8 * part_n));
   p.und      = reinterpret_cast<uint32_t*>(take(4 * words));
   p.vis_a    = reinterpret_cast<uint32_t*>(take(4 * words));
@@ -849,7 +847,7 @@ enqueue_batch(kspn_context* ctx, batch_cache& c, bt_args const& a0)
   k_bt_classify<<<cgrid < 1 ? 1 : cgrid, 256, 0, s>>>(G, a0.vtx_off, a0.fh, c.cluster_min, p.keys, p.order, p.words, p.ctr);
   KSPN_CHECK_LAUNCH();
   exclusive_scan<uint64_t>(s, f_words{ p.words }, G, p.word_off, p.part64, nullptr);
-  radix_sort_pairs(ctx, p.keys, p.order, p.kalt, p.valt, G, 0, 32, p.hist, p.part);
+  radix_sort_pairs(ctx, p.keys, p.order, p.kalt, p.valt, G, 0, 32, p.hist);
   bt_args a    = a0;
   a.word_off   = p.word_off;
   a.und        = p.und;

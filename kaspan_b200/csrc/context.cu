@@ -153,6 +153,7 @@ read_counters(kspn_context* ctx)
 {
   KSPN_CUDA(cudaMemcpyAsync(ctx->h_ctr, ctx->ws.ctr, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
   KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
+  look_back_check(ctx);
 }
 
 void
@@ -379,6 +380,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
       KSPN_CUDA(cudaMemcpyAsync(ctx->h_ctr, ws.ctr, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
       KSPN_CUDA(cudaEventRecord(ctx->ev[3], ctx->stream));
       KSPN_CUDA(cudaEventSynchronize(ctx->ev[3]));
+      look_back_check(ctx);
       if (opt.validate) validate_check(ctx->h_ctr[CTR_ERR]);
       resident_result r = fw_bw_trim_result(ctx, g, opt, st);
       if (r.resumed) {
@@ -552,7 +554,7 @@ with_transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* fh, ui
     (void)store;
     auto* nbh = reinterpret_cast<uint64_t*>(base);
     auto* nbc = reinterpret_cast<uint32_t*>(base + align_up((static_cast<size_t>(n) + 1) * 8));
-    transpose(ctx, n, m, fh, fc, nbh, nbc, nullptr);
+    transpose(ctx, n, m, fh, fc, nbh, nbc);
     g.bh = nbh;
     g.bc = nbc;
   }
@@ -762,6 +764,7 @@ kspn_context_create_on_stream(int device, void* stream, kspn_context** out)
     ctx->h_ctr   = static_cast<uint32_t*>(h);
     ctx->h_ctr64 = reinterpret_cast<uint64_t*>(ctx->h_ctr + 32);
     KSPN_CUDA(cudaMallocHost(&ctx->h_state, 4096));
+    std::memset(ctx->h_state, 0, 4096);
     for (auto& e : ctx->ev) KSPN_CUDA(cudaEventCreate(&e));
     for (auto& e : ctx->pe) KSPN_CUDA(cudaEventCreate(&e));
   });
@@ -808,7 +811,10 @@ int
 kspn_context_synchronize(kspn_context* ctx)
 {
   if (!ctx) return KSPN_ERR_INVALID_ARGUMENT;
-  return guard(ctx, [&] { KSPN_CUDA(cudaStreamSynchronize(ctx->stream)); });
+  return guard(ctx, [&] {
+    KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
+    look_back_check(ctx);
+  });
 }
 
 uint64_t
@@ -1311,7 +1317,7 @@ kspn_transpose(kspn_context* ctx, uint32_t n, uint64_t m, const uint64_t* d_fw_h
   return guard(ctx, [&] {
     require(d_fw_head && d_bw_head && (m == 0 || (d_fw_csr && d_bw_csr)), "null pointer");
     bind_device(ctx);
-    transpose(ctx, n, m, d_fw_head, d_fw_csr, d_bw_head, d_bw_csr, nullptr);
+    transpose(ctx, n, m, d_fw_head, d_fw_csr, d_bw_head, d_bw_csr);
   });
 }
 
@@ -1325,6 +1331,7 @@ kspn_upload_transpose(kspn_context* ctx, uint32_t n, uint64_t m, const uint64_t*
     bind_device(ctx);
     upload_transpose(ctx, n, m, fw_head, fw_csr, d_fw_head, d_fw_csr, d_bw_head, d_bw_csr, chunk_edges);
     KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
+    look_back_check(ctx);
   });
 }
 

@@ -43,40 +43,142 @@ k_expand_rows(uint32_t n, uint64_t const* __restrict__ head, uint32_t* __restric
 // head[v] = first index of key v in the ascending keys[0, m) (= m past the
 // last key): every boundary between two different keys writes the heads of
 // the ids it spans, so each head is written exactly once, without atomics.
-__global__ void
+// A stream of 4 m + 8 n bytes: four keys per 16-byte load (keys starts on a
+// 16-byte boundary), the one before them from the lane below.
+__global__ void __launch_bounds__(256)
 k_heads_from_sorted(uint32_t n, uint64_t m, uint32_t const* __restrict__ keys, uint64_t* __restrict__ head)
 {
+  unsigned const lane   = threadIdx.x & 31u;
   uint64_t const stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i <= m; i += stride) {
+  uint64_t const quads  = m / 4 + 1; // quad q: the boundaries before entries 4q .. 4q + 3, up to the one after the last entry
+  for (uint64_t qb = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x - lane; qb < quads; qb += stride) {
+    uint64_t const q  = qb + lane;
+    uint64_t const i0 = q * 4;
     // ids >= n (an invalid graph, reported by validation afterwards) are
-    // clamped so that no head beyond n is written
-    int64_t const lo = i == 0 ? -1 : static_cast<int64_t>(min(keys[i - 1], n));
-    int64_t const hi = i == m ? static_cast<int64_t>(n) : static_cast<int64_t>(min(keys[i], n));
-    for (int64_t v = lo + 1; v <= hi; ++v) head[v] = i;
+    // clamped so that no head beyond n is written; past the end: n
+    uint32_t k[4] = { n, n, n, n };
+    if (i0 + 4 <= m) {
+      uint4 const x = *reinterpret_cast<uint4 const*>(keys + i0);
+      k[0] = min(x.x, n), k[1] = min(x.y, n), k[2] = min(x.z, n), k[3] = min(x.w, n);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i0 + j < m) k[j] = min(keys[i0 + j], n);
+    }
+    uint32_t const below = __shfl_up_sync(0xFFFFFFFFu, k[3], 1);
+    int64_t        lo    = lane ? below : (i0 == 0 ? -1 : static_cast<int64_t>(i0 <= m ? min(keys[i0 - 1], n) : n));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (i0 + j <= m)
+        for (int64_t v = lo + 1; v <= static_cast<int64_t>(k[j]); ++v) head[v] = i0 + j;
+      lo = k[j];
+    }
   }
 }
 
-// keep[i] = 1 for the first copy of each (src, dst) with src != dst
-struct f_keep
-{
-  uint32_t const* s;
-  uint32_t const* d;
-  __device__ uint32_t operator()(uint64_t i) const
-  {
-    if (s[i] == d[i]) return 0u;
-    if (i > 0 && s[i - 1] == s[i] && d[i - 1] == d[i]) return 0u;
-    return 1u;
-  }
-};
+// ---------------------------------------------------------------- sorted edges -> CSR
+// (s, d)[0, m_raw) sorted by (s, d): self-loops and repeats are dropped, the
+// rest become csr, and head[v] = edges kept before v's first edge.  Chunk c
+// of the list belongs to block c of both kernels: k_edges_count counts its
+// kept edges, k_edges_to_csr adds up the counts before its own (at most
+// ET_CHUNKS of them, in L2) and writes.  Two reads of the list (16 B per raw
+// edge) instead of one, but no chunk waits for another: with a decoupled
+// look-back the one-pass form took 580 us on the scale-22 R-MAT edge list
+// (64 M edges), and a scan of the keep flags into positions, a compaction
+// and a pass over the kept sources 1,085 us.  build_csr of that list, both
+// sorts included: 6.1 -> 2.95 ms; its transpose 2.8 -> 1.39 ms.
+constexpr int      ET_THREADS = 256, ET_ITEMS = 4, ET_TILE = ET_THREADS * ET_ITEMS, ET_WARPS = ET_THREADS / 32;
+constexpr uint32_t ET_CHUNKS  = 148 * 8;
 
-__global__ void
-k_compact_edges(uint64_t m_raw, uint32_t const* __restrict__ s, uint32_t const* __restrict__ d, uint32_t const* __restrict__ pos, uint32_t* __restrict__ csr, uint32_t* __restrict__ src_kept)
+// Edge i = (sv, dv) (all lanes of the warp call it, lane l with edge i0 + l):
+// is it kept, and the source before it in ps (~0 for the first edge).
+__device__ __forceinline__ bool
+edge_kept(uint32_t const* s, uint32_t const* d, uint64_t i, uint32_t sv, uint32_t dv, uint32_t& ps)
 {
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < m_raw; i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-    if (pos[i + 1] != pos[i]) {
-      csr[pos[i]]      = d[i];
-      src_kept[pos[i]] = s[i];
+  uint32_t pd = __shfl_up_sync(0xFFFFFFFFu, dv, 1);
+  ps          = __shfl_up_sync(0xFFFFFFFFu, sv, 1);
+  if ((threadIdx.x & 31u) == 0 && i > 0) ps = s[i - 1], pd = d[i - 1];
+  if (i == 0) ps = 0xFFFFFFFFu;
+  return sv != dv && !(i > 0 && ps == sv && pd == dv);
+}
+
+__global__ void __launch_bounds__(ET_THREADS, 8)
+k_edges_count(uint64_t m_raw, uint64_t chunk, uint32_t const* __restrict__ s, uint32_t const* __restrict__ d, uint32_t* __restrict__ cnt)
+{
+  uint64_t const lo = blockIdx.x * chunk, hi = min(m_raw, lo + chunk);
+  uint32_t       c = 0;
+  for (uint64_t base = lo; base < hi; base += ET_TILE) {
+    uint32_t sv[ET_ITEMS], dv[ET_ITEMS], ps;
+#pragma unroll
+    for (int r = 0; r < ET_ITEMS; ++r) {
+      uint64_t const i = base + r * ET_THREADS + threadIdx.x;
+      sv[r] = dv[r] = 0; // not kept
+      if (i < hi) sv[r] = s[i], dv[r] = d[i];
     }
+#pragma unroll
+    for (int r = 0; r < ET_ITEMS; ++r) {
+      uint64_t const i = base + r * ET_THREADS + threadIdx.x;
+      c += edge_kept(s, d, i < hi ? i : 0, sv[r], dv[r], ps);
+    }
+  }
+  uint32_t total;
+  block_exclusive_scan<uint32_t, ET_THREADS>(c, &total);
+  if (threadIdx.x == 0) cnt[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(ET_THREADS, 8)
+k_edges_to_csr(uint32_t n, uint64_t m_raw, uint64_t chunk, uint32_t const* __restrict__ s, uint32_t const* __restrict__ d, uint32_t const* __restrict__ cnt, uint32_t* __restrict__ csr,
+               uint64_t* __restrict__ head, uint32_t* __restrict__ m_out)
+{
+  __shared__ uint32_t s_cnt[2][ET_ITEMS * ET_WARPS]; // kept edges per (row of ET_THREADS edges, warp); tiles alternate
+  static_assert(ET_ITEMS * ET_WARPS == 32, "one count per lane");
+  unsigned const t = threadIdx.x, w = t >> 5, lane = t & 31u, lt = (1u << lane) - 1u;
+  uint64_t const lo = blockIdx.x * chunk, hi = min(m_raw, lo + chunk);
+  uint32_t       sum = 0, before; // kept edges before the tile: below m_raw < 2^32
+  for (uint32_t k = t; k < blockIdx.x; k += ET_THREADS) sum += cnt[k];
+  block_exclusive_scan<uint32_t, ET_THREADS>(sum, &before);
+  int flip = 0;
+  for (uint64_t base = lo; base < hi; base += ET_TILE, flip ^= 1) {
+    uint32_t sv[ET_ITEMS], dv[ET_ITEMS], ps[ET_ITEMS];
+    unsigned keep[ET_ITEMS];
+#pragma unroll
+    for (int r = 0; r < ET_ITEMS; ++r) {
+      uint64_t const i = base + r * ET_THREADS + t;
+      sv[r] = dv[r] = 0;
+      if (i < hi) sv[r] = s[i], dv[r] = d[i];
+    }
+#pragma unroll
+    for (int r = 0; r < ET_ITEMS; ++r) {
+      uint64_t const i = base + r * ET_THREADS + t;
+      keep[r]          = __ballot_sync(0xFFFFFFFFu, edge_kept(s, d, i < hi ? i : 0, sv[r], dv[r], ps[r]));
+      if (lane == 0) s_cnt[flip][r * ET_WARPS + w] = __popc(keep[r]);
+    }
+    __syncthreads();
+    uint32_t const mine = s_cnt[flip][lane]; // every warp scans the counts for itself
+    uint32_t       incl = mine;
+#pragma unroll
+    for (int dd = 1; dd < 32; dd <<= 1) {
+      uint32_t const y = __shfl_up_sync(0xFFFFFFFFu, incl, dd);
+      if (lane >= static_cast<unsigned>(dd)) incl += y;
+    }
+#pragma unroll
+    for (int r = 0; r < ET_ITEMS; ++r) {
+      uint64_t const i   = base + r * ET_THREADS + t;
+      uint32_t const pos = before + __shfl_sync(0xFFFFFFFFu, incl - mine, r * ET_WARPS + w) + __popc(keep[r] & lt);
+      uint32_t const k   = (keep[r] >> lane) & 1u;
+      if (k) csr[pos] = dv[r];
+      if (i < hi && (ps[r] != sv[r] || i == 0 || i + 1 == m_raw)) {
+        // the rows that start at this edge (ids >= n, an invalid list, are
+        // clamped), and after the last edge the rows past it
+        uint32_t const up = min(sv[r], n);
+        for (uint64_t v = i == 0 ? 0 : static_cast<uint64_t>(min(ps[r], n)) + 1; v <= up; ++v) head[v] = pos;
+        if (i + 1 == m_raw) {
+          for (uint64_t v = static_cast<uint64_t>(up) + 1; v <= n; ++v) head[v] = pos + k;
+          *m_out = pos + k;
+        }
+      }
+    }
+    before += __shfl_sync(0xFFFFFFFFu, incl, 31);
   }
 }
 
@@ -349,7 +451,7 @@ alloc_scratch(kspn_context* ctx, scratch& s, size_t bytes)
 } // namespace
 
 void
-transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* fh, uint32_t const* fc, uint64_t* bh, uint32_t* bc, uint32_t* /*unused*/)
+transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* fh, uint32_t const* fc, uint64_t* bh, uint32_t* bc)
 {
   cudaStream_t const s = ctx->stream;
   if (n == 0) {
@@ -357,29 +459,27 @@ transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* fh, uint32_
     return;
   }
   size_t const hist_n = radix_hist_entries(m);
-  size_t const part_n = scan_partial_entries(hist_n > n + 1 ? hist_n : n + 1);
   scratch      sc;
-  alloc_scratch(ctx, sc, 3 * (m + 64) * sizeof(uint32_t) + (hist_n + part_n + n + 64) * sizeof(uint64_t) + 4096);
-  size_t    off   = 0;
-  uint32_t* keys  = sc.carve<uint32_t>(off, m + 1);
-  uint32_t* kalt  = sc.carve<uint32_t>(off, m + 1);
-  uint32_t* valt  = sc.carve<uint32_t>(off, m + 1);
-  uint32_t* hist  = sc.carve<uint32_t>(off, hist_n);
-  uint32_t* part  = sc.carve<uint32_t>(off, part_n);
-  uint32_t* cnt   = sc.carve<uint32_t>(off, n + 1);
-  uint64_t* part64 = sc.carve<uint64_t>(off, part_n);
+  alloc_scratch(ctx, sc, (3 * (m + 64) + hist_n) * sizeof(uint32_t) + 4096);
+  size_t    off  = 0;
+  uint32_t* ka   = sc.carve<uint32_t>(off, m + 1);
+  uint32_t* kb   = sc.carve<uint32_t>(off, m + 1);
+  uint32_t* va   = sc.carve<uint32_t>(off, m + 1);
+  uint32_t* hist = sc.carve<uint32_t>(off, hist_n);
 
+  // (target, source) pairs sorted by target, read where the targets lie,
+  // through A = (ka, va) and B = (kb, bc); the last pass writes B, so the
+  // sources start in the value buffer that the first pass does not write
+  int const passes = m ? radix_passes(0, bits_for(n)) : 0;
   if (m) {
-    KSPN_CUDA(cudaMemcpyAsync(keys, fc, m * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-    k_expand_rows<<<div_up(n, 256), 256, 0, s>>>(n, fh, bc);
+    uint32_t* const src = passes % 2 ? va : bc;
+    k_expand_rows<<<div_up(n, 256), 256, 0, s>>>(n, fh, src);
     KSPN_CHECK_LAUNCH();
-    radix_sort_pairs(ctx, keys, bc, kalt, valt, m, 0, bits_for(n), hist, part);
+    radix_sort_pairs_to(ctx, fc, src, kb, bc, ka, va, kb, bc, m, bits_for(n), hist);
   }
-  k_heads_from_sorted<<<grid_for(m + 1, 256), 256, 0, s>>>(n, m, keys, bh);
+  k_heads_from_sorted<<<grid_for(m / 4 + 1, 256), 256, 0, s>>>(n, m, kb, bh);
   KSPN_CHECK_LAUNCH();
   ctx->launches += 2;
-  (void)cnt;
-  (void)part64;
 }
 
 namespace {
@@ -412,10 +512,10 @@ upload_transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* h_fh
   // the chunk row ranges come from binary searches over the host offsets
   if (h_fh[0] != 0 || h_fh[n] != m) throw error{ KSPN_ERR_INVALID_GRAPH, "invalid graph: head[0] != 0 or head[n] != m;" };
   size_t const hist_n = radix_hist_entries(chunk);
-  size_t const part_n = scan_partial_entries((hist_n > n + 1 ? hist_n : n + 1));
+  size_t const part_n = scan_partial_entries(static_cast<uint64_t>(n) + 1);
   scratch      sc;
   size_t const band_cap = (BAND_MAX + 1) * ((m + chunk - 1) / chunk);
-  alloc_scratch(ctx, sc, (3 * (m + 64) + 5 * (chunk + 64) + (static_cast<size_t>(n) + 64) + BAND_MAX + 64 + band_cap + 64) * sizeof(uint32_t) + (hist_n + part_n) * sizeof(uint32_t) + part_n * sizeof(uint64_t) + 16384);
+  alloc_scratch(ctx, sc, (3 * (m + 64) + 5 * (chunk + 64) + (static_cast<size_t>(n) + 64) + BAND_MAX + 64 + band_cap + 64 + hist_n) * sizeof(uint32_t) + part_n * sizeof(uint64_t) + 16384);
   size_t    off    = 0;
   uint32_t* skeys  = sc.carve<uint32_t>(off, m);     // chunk-sorted targets
   uint32_t* svals  = sc.carve<uint32_t>(off, m);     // their sources
@@ -427,7 +527,6 @@ upload_transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* h_fh
   uint32_t* vb     = sc.carve<uint32_t>(off, chunk);
   uint32_t* indeg  = sc.carve<uint32_t>(off, n);
   uint32_t* hist   = sc.carve<uint32_t>(off, hist_n);
-  uint32_t* part   = sc.carve<uint32_t>(off, part_n);
   uint64_t* part64 = sc.carve<uint64_t>(off, part_n);
   uint32_t* bv     = sc.carve<uint32_t>(off, BAND_MAX + 1);
   uint32_t* seg    = sc.carve<uint32_t>(off, band_cap);
@@ -444,7 +543,7 @@ upload_transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* h_fh
     uint32_t const u_hi = static_cast<uint32_t>(std::lower_bound(h_fh + u_lo, h_fh + n + 1, e1) - h_fh);
     k_expand_range<<<div_up(static_cast<uint64_t>(u_hi - u_lo), 256), 256, 0, s>>>(u_lo, u_hi, dfh, e0, e1, src);
     KSPN_CHECK_LAUNCH();
-    radix_sort_pairs_to(ctx, dfc + e0, src, skeys + e0, svals + e0, ka, va, kb, vb, cnt, bits, hist, part);
+    radix_sort_pairs_to(ctx, dfc + e0, src, skeys + e0, svals + e0, ka, va, kb, vb, cnt, bits, hist);
     unsigned const g = grid_for(cnt, 256);
     k_run_offsets<<<div_up(cnt, RO_THREADS * RO_ITEMS), RO_THREADS, 0, s>>>(n, skeys + e0, cnt, indeg, roff + e0);
     k_run_ends<<<g, 256, 0, s>>>(n, skeys + e0, cnt, roff + e0, indeg);
@@ -474,39 +573,37 @@ build_csr(kspn_context* ctx, uint32_t n, uint64_t m_raw, uint32_t* src, uint32_t
 {
   cudaStream_t const s = ctx->stream;
   if (m_raw >= 0xFFFFFFFFull) throw error{ KSPN_ERR_INVALID_ARGUMENT, "build_csr: edge lists of 2^32-1 or more entries are not supported" };
-  size_t const hist_n = radix_hist_entries(m_raw);
-  size_t const part_n = scan_partial_entries((hist_n > m_raw + 1 ? hist_n : m_raw + 1) + n + 1);
-  scratch      sc;
-  alloc_scratch(ctx, sc, 3 * (m_raw + 64) * sizeof(uint32_t) + (hist_n + part_n + n + 64) * sizeof(uint64_t) + 4096);
-  size_t    off    = 0;
-  uint32_t* kalt   = sc.carve<uint32_t>(off, m_raw + 1);
-  uint32_t* valt   = sc.carve<uint32_t>(off, m_raw + 1);
-  uint32_t* pos    = sc.carve<uint32_t>(off, m_raw + 1);
-  uint32_t* hist   = sc.carve<uint32_t>(off, hist_n);
-  uint32_t* part   = sc.carve<uint32_t>(off, part_n);
-  uint32_t* rowcnt = sc.carve<uint32_t>(off, n + 1);
-  uint64_t* part64 = sc.carve<uint64_t>(off, part_n);
-
-  int const b = bits_for(n);
-  // (dst, src) stably by dst, then (src, dst) stably by src => sorted by (src, dst)
-  radix_sort_pairs(ctx, dst, src, kalt, valt, m_raw, 0, b, hist, part);
-  radix_sort_pairs(ctx, src, dst, kalt, valt, m_raw, 0, b, hist, part);
-  exclusive_scan<uint32_t>(s, f_keep{ src, dst }, m_raw, pos, part, &ctx->launches);
-  uint32_t m32 = 0;
-  KSPN_CUDA(cudaMemcpyAsync(&m32, pos + m_raw, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  KSPN_CUDA(cudaStreamSynchronize(s));
-  uint64_t const m = m32;
-  if (m_raw) {
-    k_compact_edges<<<grid_for(m_raw, 256), 256, 0, s>>>(m_raw, src, dst, pos, csr, kalt);
-    KSPN_CHECK_LAUNCH();
-    ctx->launches += 1;
+  if (m_raw == 0) {
+    KSPN_CUDA(cudaMemsetAsync(head, 0, (static_cast<size_t>(n) + 1) * sizeof(uint64_t), s));
+    KSPN_CUDA(cudaStreamSynchronize(s));
+    return 0;
   }
-  k_heads_from_sorted<<<grid_for(m + 1, 256), 256, 0, s>>>(n, m, kalt, head);
+  size_t const hist_n = radix_hist_entries(m_raw);
+  scratch      sc;
+  alloc_scratch(ctx, sc, (2 * (m_raw + 64) + hist_n) * sizeof(uint32_t) + 4096);
+  size_t    off  = 0;
+  uint32_t* dalt = sc.carve<uint32_t>(off, m_raw + 1);
+  uint32_t* salt = sc.carve<uint32_t>(off, m_raw + 1);
+  uint32_t* hist = sc.carve<uint32_t>(off, hist_n);
+
+  // (dst, src) stably by dst, then (src, dst) stably by src => sorted by
+  // (src, dst); each sort goes on from the buffers the last pass wrote
+  int const b = bits_for(n);
+  if (radix_sort_alternate(ctx, dst, src, dalt, salt, m_raw, 0, b, hist)) std::swap(dst, dalt), std::swap(src, salt);
+  if (radix_sort_alternate(ctx, src, dst, salt, dalt, m_raw, 0, b, hist)) std::swap(dst, dalt), std::swap(src, salt);
+  // chunks of whole tiles, one block each
+  uint64_t const chunk  = (div_up(m_raw, ET_TILE) + ET_CHUNKS - 1) / ET_CHUNKS * ET_TILE;
+  unsigned const chunks = div_up(m_raw, chunk);
+  uint32_t*      cnt    = hist; // ET_CHUNKS counts and the total (the sort's scratch is larger)
+  static_assert(ET_CHUNKS + 1 <= 1500, "counts must fit the smallest sort scratch");
+  k_edges_count<<<chunks, ET_THREADS, 0, s>>>(m_raw, chunk, src, dst, cnt);
+  k_edges_to_csr<<<chunks, ET_THREADS, 0, s>>>(n, m_raw, chunk, src, dst, cnt, csr, head, cnt + ET_CHUNKS);
   KSPN_CHECK_LAUNCH();
-  ctx->launches += 1;
-  (void)rowcnt;
-  (void)part64;
+  ctx->launches += 2;
+  uint32_t m = 0;
+  KSPN_CUDA(cudaMemcpyAsync(&m, cnt + ET_CHUNKS, sizeof(m), cudaMemcpyDeviceToHost, s));
   KSPN_CUDA(cudaStreamSynchronize(s));
+  look_back_check(ctx);
   return m;
 }
 

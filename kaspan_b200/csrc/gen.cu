@@ -229,10 +229,10 @@ gen_rgg(kspn_context* ctx, uint32_t n, uint64_t seed, uint32_t g, uint64_t r2, u
   uint64_t const cells = static_cast<uint64_t>(g) * g;
   if (cells >= 0xFFFFFFFFull) throw error{ KSPN_ERR_INVALID_ARGUMENT, "gen_rgg: g * g must be below 2^32 - 1" };
   size_t const hist_n = radix_hist_entries(n);
-  size_t const part_n = scan_partial_entries((hist_n > n + 1 ? hist_n : n + 1) + 1);
-  // scratch: cell, idx (+ alternates), radix histogram + partials, points,
+  size_t const part_n = scan_partial_entries(static_cast<uint64_t>(n) + 2);
+  // scratch: cell, idx (+ alternates), radix scratch, points,
   // cell starts, per-vertex counts and edge offsets
-  size_t const bytes = (6 * (static_cast<size_t>(n) + 64) + hist_n + part_n) * sizeof(uint32_t) + (cells + 1 + n + 1 + part_n + 256) * sizeof(uint64_t) + 16 * 256;
+  size_t const bytes = (6 * (static_cast<size_t>(n) + 64) + hist_n) * sizeof(uint32_t) + (cells + 1 + n + 1 + part_n + 256) * sizeof(uint64_t) + 16 * 256;
   char*        base  = static_cast<char*>(context_buffer(ctx, BUF_GEN, bytes));
   size_t       off   = 0;
   auto         take  = [&](size_t count, size_t elem) {
@@ -248,7 +248,6 @@ gen_rgg(kspn_context* ctx, uint32_t n, uint64_t seed, uint32_t g, uint64_t r2, u
   auto* px        = static_cast<uint32_t*>(take(n + 1, 4));
   auto* py        = static_cast<uint32_t*>(take(n + 1, 4));
   auto* hist      = static_cast<uint32_t*>(take(hist_n, 4));
-  auto* part      = static_cast<uint32_t*>(take(part_n, 4));
   auto* cstart    = static_cast<uint64_t*>(take(cells + 1, 8));
   auto* offs      = static_cast<uint64_t*>(take(static_cast<size_t>(n) + 1, 8));
   auto* part64    = static_cast<uint64_t*>(take(part_n, 8));
@@ -258,7 +257,7 @@ gen_rgg(kspn_context* ctx, uint32_t n, uint64_t seed, uint32_t g, uint64_t r2, u
   unsigned const grid = gen_grid(n);
   k_rgg_points<<<grid, 256, 0, s>>>(n, key, g, cell, idx);
   KSPN_CHECK_LAUNCH();
-  if (cells > 1) radix_sort_pairs(ctx, cell, idx, cell_alt, idx_alt, n, 0, bits_for(cells), hist, part);
+  if (cells > 1) radix_sort_pairs(ctx, cell, idx, cell_alt, idx_alt, n, 0, bits_for(cells), hist);
   k_rgg_gather<<<grid, 256, 0, s>>>(n, key, idx, px, py);
   k_rgg_cells<<<gen_grid(static_cast<uint64_t>(n) + 1), 256, 0, s>>>(cells, n, cell, cstart);
   k_rgg_count<<<grid, 256, 0, s>>>(n, px, py, cstart, g, r2, key2, cnt);

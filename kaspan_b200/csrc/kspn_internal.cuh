@@ -544,7 +544,7 @@ uint32_t label_search(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_
 void canonicalise(kspn_context* ctx, uint32_t n, uint32_t* scc_id, uint32_t* scratch, bool members);
 
 // csr.cu
-void     transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* fh, uint32_t const* fc, uint64_t* bh, uint32_t* bc, uint32_t* scratch_n);
+void     transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* fh, uint32_t const* fc, uint64_t* bh, uint32_t* bc);
 // Upload of a host CSR in chunks of `chunk` edges (0: UPLOAD_CHUNK) on the
 // context's copy stream, with the CSC built on the context's stream while
 // later chunks are still in flight: each arrived chunk's (target, source)

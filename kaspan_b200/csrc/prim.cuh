@@ -152,15 +152,48 @@ struct f_frontier_degree
   }
 };
 
+// Words of a decoupled look-back: value and state in one 64-bit word, so a
+// relaxed load sees both or neither.
+__device__ __forceinline__ unsigned long long
+ld_relaxed64(unsigned long long const* p)
+{
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void
+st_relaxed64(unsigned long long* p, unsigned long long v)
+{
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// Error word of kernels with a decoupled look-back (a tile waits for earlier
+// tiles' counts, with a bound): the last word of the context's pinned state
+// mirror, which kernels reach over the unified address space.
+constexpr size_t LOOK_BACK_ERR_AT = 4092;
+inline uint32_t*
+look_back_err(kspn_context* ctx)
+{
+  return reinterpret_cast<uint32_t*>(static_cast<char*>(ctx->h_state) + LOOK_BACK_ERR_AT);
+}
+// After the stream was synchronised: throws if a look-back gave up.
+void look_back_check(kspn_context* ctx);
+
 // radix.cu: stable LSD radix sort of (key, value) u32 pairs on key bits
 // [begin_bit, end_bit).  The result ends in keys/vals; keys_alt/vals_alt
 // are scratch of the same size.  hist needs radix_hist_entries(count).
 size_t radix_hist_entries(uint64_t count);
-void   radix_sort_pairs(kspn_context* ctx, uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint64_t count, int begin_bit, int end_bit, uint32_t* hist, uint32_t* hist_partial);
+int    radix_passes(int begin_bit, int end_bit); // passes over the pairs such a sort makes
+void   radix_sort_pairs(kspn_context* ctx, uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint64_t count, int begin_bit, int end_bit, uint32_t* hist);
+// The same, leaving the result where the last pass put it: true = in
+// keys_alt/vals_alt (after an odd number of passes).
+bool   radix_sort_alternate(kspn_context* ctx, uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint64_t count, int begin_bit, int end_bit, uint32_t* hist);
 // The same sort on key bits [0, end_bit) from read-only input (kin, vin) to
-// (kout, vout); (ka, va) and (kb, vb) are scratch of `count` entries each
-// (neither may alias the input or the output).
-void   radix_sort_pairs_to(kspn_context* ctx, uint32_t const* kin, uint32_t const* vin, uint32_t* kout, uint32_t* vout, uint32_t* ka, uint32_t* va, uint32_t* kb, uint32_t* vb, uint64_t count, int end_bit, uint32_t* hist, uint32_t* hist_partial);
+// (kout, vout); (ka, va) and (kb, vb) are scratch of `count` entries each.
+// Pass p of P writes A when P - 1 - p is odd and B when it is even and not
+// the last; no pass may read a buffer it writes, so an output or the input
+// may share memory with a scratch buffer of the other parity only.
+void   radix_sort_pairs_to(kspn_context* ctx, uint32_t const* kin, uint32_t const* vin, uint32_t* kout, uint32_t* vout, uint32_t* ka, uint32_t* va, uint32_t* kb, uint32_t* vb, uint64_t count, int end_bit, uint32_t* hist);
 
 inline int
 bits_for(uint64_t n) // bits needed to represent ids in [0, n)

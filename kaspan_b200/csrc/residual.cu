@@ -356,7 +356,7 @@ residual(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, ui
   KSPN_CUDA(cudaStreamSynchronize(s));
   ctx->launches += 6;
   if (k == 0) return 0;
-  radix_sort_pairs(ctx, keys, vals, kalt, valt, k, 0, bits_for(g.n), hist, part);
+  radix_sort_pairs(ctx, keys, vals, kalt, valt, k, 0, bits_for(g.n), hist);
   exclusive_scan<uint32_t>(s, f_seg_head{ keys }, k, spos, part, &ctx->launches);
   k_res_segments<<<rs_grid(k), RS_THREADS, 0, s>>>(k, keys, spos, seg);
   // pieces: spos[k] of them, starts in seg
