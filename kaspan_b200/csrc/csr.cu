@@ -580,7 +580,10 @@ build_csr(kspn_context* ctx, uint32_t n, uint64_t m_raw, uint32_t* src, uint32_t
   }
   size_t const hist_n = radix_hist_entries(m_raw);
   scratch      sc;
-  alloc_scratch(ctx, sc, (2 * (m_raw + 64) + hist_n) * sizeof(uint32_t) + 4096);
+  // a third edge array that only the transpose needs: a caller who goes on
+  // with it finds its scratch there, instead of freeing this one for a larger
+  // one after the caller's own allocations have taken what is left
+  alloc_scratch(ctx, sc, (3 * (m_raw + 64) + hist_n) * sizeof(uint32_t) + 4096);
   size_t    off  = 0;
   uint32_t* dalt = sc.carve<uint32_t>(off, m_raw + 1);
   uint32_t* salt = sc.carve<uint32_t>(off, m_raw + 1);
