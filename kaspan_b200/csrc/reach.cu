@@ -434,12 +434,15 @@ bu_sweep_chunk(uint32_t c,
 // (independent loads); the chunks are then taken in segments of at most
 // 32 x 32 candidates (the pack buffer), each packed once and walked in
 // batches of 32 x BU_ILP as bu_rows does, after which lane i writes back
-// word i of each chunk of the segment.  On a sparse level one segment holds
+// word i of each chunk of the segment.  A chunk is cw words (32, fewer on a
+// graph of too few words to give every warp of the grid one, then cnt = 1).
+// On a sparse level one segment holds
 // the whole group, so its few candidates share one dependent head ->
 // neighbour -> probe chain instead of one chain per chunk.
 __device__ __forceinline__ void
 bu_sweep_group(uint32_t c0,
                uint32_t cnt,
+               uint32_t cw,
                uint32_t n,
                uint64_t const* __restrict__ head,
                uint32_t const* __restrict__ adj,
@@ -458,8 +461,8 @@ bu_sweep_group(uint32_t c0,
   // segment is packed (no register array across the scans)
 #pragma unroll
   for (int g = 0; g < BU_GROUP; ++g) {
-    uint32_t const w = (c0 + g) * 32 + lane;
-    uint32_t       x = static_cast<uint32_t>(g) < cnt && w < words ? __ldcg(avail + w) : 0u;
+    uint32_t const w = (c0 + g) * cw + lane;
+    uint32_t       x = static_cast<uint32_t>(g) < cnt && lane < cw && w < words ? __ldcg(avail + w) : 0u;
     if (w == words - 1 && (n & 31)) x &= (1u << (n & 31)) - 1u;
     sm.found[g * 32 + lane] = x;
   }
@@ -493,7 +496,7 @@ bu_sweep_group(uint32_t c0,
     }
     __syncwarp();
     ncand += lane == 0 ? total : 0;
-    uint32_t const vbase = (c0 + s0) * 1024;
+    uint32_t const vbase = (c0 + s0) * cw * 32;
     for (uint32_t r = 0; r < total; r += 32 * BU_ILP) {
       uint32_t v[BU_ILP];
       bool     live[BU_ILP], found[BU_ILP];
@@ -506,13 +509,13 @@ bu_sweep_group(uint32_t c0,
       bu_rows(v, live, found, head, adj, mark, cut, nedge);
 #pragma unroll
       for (int k = 0; k < BU_ILP; ++k)
-        if (found[k]) atomicOr(&sm.found[(v[k] >> 5) - c0 * 32], 1u << (v[k] & 31));
+        if (found[k]) atomicOr(&sm.found[(v[k] >> 5) - c0 * cw], 1u << (v[k] & 31));
     }
     __syncwarp();
     for (uint32_t g = s0; g < s1; ++g) {
-      uint32_t const w   = (c0 + g) * 32 + lane;
+      uint32_t const w   = (c0 + g) * cw + lane;
       uint32_t const fnd = sm.found[g * 32 + lane];
-      if (w < words) {
+      if (lane < cw && w < words) {
         if (fnd) {
           atomicAnd(avail + w, ~fnd);
           atomicOr(mark + w, fnd);
@@ -524,6 +527,20 @@ bu_sweep_group(uint32_t c0,
     __syncwarp();
     s0 = s1;
   }
+}
+
+// Words per chunk of a bottom-up level: 32, or the power of two below that
+// gives each of the grid's warps a chunk when both searches sweep.  A warp
+// walks its chunk's candidates 32 x BU_ILP at a time, each batch one chain
+// of dependent loads: on G(n, m) of 2^16 vertices (64 chunks of 32 words, the
+// other warps idle) the first sweep took 98 us and a whole call 272 us, with
+// small chunks 191 us; on 1000 vertices (one chunk) 243 and 171 us.
+__device__ __forceinline__ uint32_t
+bu_chunk_words(uint32_t words)
+{
+  uint32_t cw = 32;
+  while (cw > 1 && words / cw * 2 < gridDim.x * BU_WARPS) cw /= 2;
+  return cw;
 }
 
 // Chunks per sweep group for a bottom-up level over `cand` candidates of n
@@ -1344,6 +1361,7 @@ struct jctl
   uint32_t           lvl[2], bu[2], mode[2], mat[2], fixed[2], live[2], kind[2];
   uint32_t           restrict_to[2]; // 1: cut this search's candidates down to the other's set first
   uint32_t           capped, async, any_td, any_bu;
+  uint32_t           cw;          // words per bottom-up chunk (bu_chunk_words)
   uint32_t           cnt[2];
 };
 __shared__ jctl s_j;
@@ -1371,6 +1389,7 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
     s_bu_cut[0] = bu_cut{ a.cutmap, a.heavy + 3u * a.heavy_cap, &st->cut_n[0], a.heavy_cap, &st->heavy_err };
     s_bu_cut[1] = bu_cut{ a.cutmap + a.cut_words, a.heavy, &st->cut_n[1], a.heavy_cap, &st->heavy_err };
     if (resume) s_j = static_cast<joint_save const*>(a.jsave)->j;
+    s_j.cw = bu_chunk_words(words);
     for (int d = 0; d < 2 && !resume; ++d) {
       uint64_t const* h = d ? a.bh : a.fh;
       s_j.c[d]          = (static_cast<unsigned long long>(h[pivot + 1] - h[pivot]) << a.qbits) | 1u; // the pivot alone
@@ -1442,7 +1461,7 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
           if (s_j.mat[d]) s_j.mode[d] = 0;
           else if (s_j.mode[d] == 0 && mf * a.alpha > s_j.m_u[d]) s_j.mode[d] = 1;
           s_j.kind[d] = s_j.mode[d] ? JK_BU : JK_TD;
-          s_j.grp[d]  = s_j.mode[d] ? bu_group_size(n_und > s_j.seen[d] ? n_und - s_j.seen[d] : 0, a.n) : 1u;
+          s_j.grp[d]  = s_j.mode[d] && s_j.cw == 32 ? bu_group_size(n_und > s_j.seen[d] ? n_und - s_j.seen[d] : 0, a.n) : 1u;
           if (!(s_j.mode[d] == 0 && s_j.lvl[d] >= ASYNC_AFTER && qn <= ASYNC_FRONTIER)) async = false;
         }
         s_j.async  = async && live && !s_j.capped;
@@ -1576,7 +1595,8 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
     if (s_j.any_bu) {
       // both searches' chunks (or sparse groups of chunks) in one range,
       // spread over every warp of the grid
-      uint32_t const chunks = (words + 31) / 32;
+      uint32_t const cw     = s_j.cw;
+      uint32_t const chunks = (words + cw - 1) / cw;
       uint32_t const g0     = s_j.grp[0], g1 = s_j.grp[1];
       uint32_t const c0     = s_j.kind[0] == JK_BU ? (chunks + g0 - 1) / g0 : 0u;
       uint32_t const c1     = s_j.kind[1] == JK_BU ? (chunks + g1 - 1) / g1 : 0u;
@@ -1588,7 +1608,7 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
         uint32_t const gs = d ? g1 : g0;
         uint32_t const ch = (d ? cc - c0 : cc) * gs;
         uint32_t       f  = 0;
-        bu_sweep_group(ch, chunks - ch < gs ? chunks - ch : gs, a.n, D.bu_head, D.bu_adj, D.avail, D.mark, D.fresh, s_bu_cut[d], sm.warp[wid], f, ne, ncd);
+        bu_sweep_group(ch, chunks - ch < gs ? chunks - ch : gs, cw, a.n, D.bu_head, D.bu_adj, D.avail, D.mark, D.fresh, s_bu_cut[d], sm.warp[wid], f, ne, ncd);
         if (d) nf1 += f;
         else nf0 += f;
       }
