@@ -84,6 +84,7 @@ layout(workspace& ws, char* base, uint32_t n, uint64_t m)
   ws.tile_zero         = c.take<uint32_t>(m / 2048 + 4);
   ws.seed_q            = c.take<uint32_t>(4);
   ws.seed_prefix       = c.take<uint64_t>(4);
+  ws.links             = c.take<uint32_t>(4096);
   ws.gbar              = c.take<char>(4096);
   ws.heavy_cap         = heavy_capacity(n, m);
   ws.aw_entries        = 4 * nn + 2 * AW_STALE + 4 * (m / HEAVY_SLICE) + 128; // see run_async: half for duplicates, the passes around the switch, one winning item per vertex and direction, the heavy-row slices

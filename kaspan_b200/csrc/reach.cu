@@ -691,6 +691,10 @@ k_bu_cut_clear(gate g, bu_cut cut)
 // is broadcast.  Level counters rotate over three slots: level L reads slot
 // L%3, adds to (L+1)%3 and clears (L+2)%3, which no block touches again
 // until after the next barrier.
+// Vertices per start vertex of a worklist phase (run_async).  RGG of 10^6 /
+// 60,000 vertices, whole call: 2048: 1.56 / 1.07 ms, 4096: 1.51 / 0.91,
+// 8192: 1.90 / 1.34; 2^24 vertices (255 start vertices each way): the same.
+constexpr uint32_t SEED_SPAN       = 4096;
 constexpr unsigned GRID_SYNC_SPINS = 1u << 22; // default wait limit (kspn_options.wait_limit = 0)
 
 // Grid barrier with a monotonically growing counter: every block adds 1
@@ -819,6 +823,13 @@ struct fwbw_args
   uint32_t const*    gate;         // not null and *gate != 0: the input check failed, the launch does nothing
   void*              jsave;        // the level loop's saved control (handoff, resume)
   uint32_t           resume;       // 1: continue a launch that handed off, at its worklist phase
+  // several start vertices for a joint worklist phase (run_async)
+  uint32_t           seeds;        // how many (0: none; at most 255)
+  uint32_t           seed_n;       // candidates at seed_ids
+  uint32_t const*    seed_ids;     // vertices, possibly stale: taken only if both searches may still reach them
+  uint8_t*           label;        // 2 x label_n bytes: the start vertex a vertex was reached from, FW then BW
+  uint64_t           label_n;      // n rounded up to 16
+  uint32_t*          links;        // LINK_WORDS: links between start vertices, then the labels in use
 };
 
 __device__ __forceinline__ bool
@@ -1020,9 +1031,16 @@ enum : int
 // (nothing in flight can append any more); the used slots are then cleared to 0, so the worklist
 // is all zeros outside a phase.  Every wait is bounded.
 constexpr uint32_t           ASYNC_AFTER    = 16;        // top-down levels before a search may switch
+constexpr uint32_t           ASYNC_SLOW     = 8;         // the same when it grows slowly, and of the trim (a level costs 12 us however thin)
 constexpr uint32_t           ASYNC_FRONTIER = 1u << 16;  // largest frontier that switches
 constexpr unsigned long long AW_TAG         = 1ull << 32; // marks a written slot
 constexpr int                AW_BATCH       = 8;         // neighbours a lane loads at once
+// In a phase with several start vertices an item carries the label of the one
+// it was reached from (bits 54..61; its slice number then has bits 33..53,
+// enough for rows below 2^31 entries).
+constexpr unsigned long long AW_LABEL       = 255ull << 54;
+constexpr int                LINK_WORDS     = 256 * 8 + 8;
+constexpr int                LINK_VERTEX    = LINK_WORDS; // after them: the start vertices by label (UNDECIDED: label not in use)
 constexpr int                AW_WARPS       = 8;         // warps per block that take worklist items (the others wait at the phase's end)
 
 // Finds a warp keeps on its own stack (in its shared buffer) and expands in
@@ -1031,9 +1049,15 @@ constexpr int                AW_WARPS       = 8;         // warps per block that
 // claimed the slot.  Finds past AW_LOCAL_KEEP go to the worklist, where idle
 // warps pick them up.  Stack entries are items (below) with slice 0.
 constexpr uint32_t           AW_LOCAL_KEEP = 16;
+// The same with several start vertices, where most warps have work of their
+// own: more on graphs that keep them busy for long (n / AW_KEEP_SPAN, within
+// the bounds), less where a deep stack would hold back what idle warps could
+// take.  RGG, seeded phase, 16 / 32 / 64 / 192 kept: 2^24 vertices 7.6 / 5.5 /
+// 4.7 / 5.5 ms, 10^6 vertices 0.94 / 0.88 / 1.10 / 4.7 ms.
+constexpr uint32_t           AW_KEEP_MIN = 24, AW_KEEP_MAX = 64, AW_KEEP_SPAN = 1u << 17;
 constexpr unsigned long long AW_BW         = 1ull << 63; // item of the BW search of a joint phase
 constexpr unsigned long long AW_TAKEN      = 1ull << 62; // the vertex was taken when it was pushed (else its consumer takes it)
-static_assert(sizeof(bu_warp_smem) >= AW_LOCAL_KEEP * sizeof(unsigned long long), "local stack must fit the warp buffer");
+static_assert(sizeof(bu_warp_smem) >= AW_KEEP_MAX * sizeof(unsigned long long), "local stack must fit the warp buffer");
 static_assert(R_THREADS / 32 == 8 && AW_BATCH == 8, "AW_STALE counts 8 warps per block and 8 finds per lane per pass");
 
 // One search's arrays in the worklist phase: rows to walk, the candidates a
@@ -1056,9 +1080,10 @@ struct aw_sink
   unsigned long long* aw;
   unsigned long long* tail;
   uint64_t            cap;
+  uint32_t            room_for; // stack size
   __device__ __forceinline__ uint32_t reserve(uint32_t ls_n, uint32_t tot, unsigned long long& gbase, uint32_t& nloc) const
   {
-    uint32_t const room = ls_n < AW_LOCAL_KEEP ? AW_LOCAL_KEEP - ls_n : 0u;
+    uint32_t const room = ls_n < room_for ? room_for - ls_n : 0u;
     nloc                = tot < room ? tot : room;
     unsigned long long b = 0;
     if ((threadIdx.x & 31u) == 0 && tot > nloc) b = atomicAdd(tail, static_cast<unsigned long long>(tot - nloc));
@@ -1071,6 +1096,182 @@ struct aw_sink
     else if (gbase + (q - nloc) < cap) __stcg(aw + gbase + (q - nloc), item);
   }
 };
+
+// ---- several start vertices in one worklist phase
+// A long, thin search is bound by its depth: one hop after another over the
+// whole diameter (RGG 2^24: 4,868 hops from the pivot).  Reachability from
+// several vertices at once is as deep as the farthest vertex from the NEAREST
+// of them, so when both searches move to the worklist (RGG of 2^24 vertices:
+// 16.1 ms there from the pivot alone, 4.0 ms with 255 more; 10^6 vertices:
+// 3.5 -> 0.7 ms), up to 255 further
+// vertices start beside them -- trim_1_first's per-block candidates that
+// neither search has reached (seed_start) -- and every vertex keeps the label
+// of the start vertex it was reached from, per direction.  Afterwards C = FW
+// & BW is a union of whole SCCs that contains the pivot's (a vertex on a path
+// between two members is in both sets).  A vertex with FW label i and BW
+// label j shows that start vertex i reaches j; when the links found that way
+// (seed_links) put every start vertex into one strongly connected set with
+// the pivot, C is the pivot's SCC.  Otherwise the sets restart inside C
+// (seed_restart): FW as the vertices whose FW label the pivot is known to
+// reach, BW as the ones whose BW label is known to reach the pivot, and both
+// searches go on among the other vertices of C from a bottom-up sweep until
+// nothing joins.  Both ways FW & BW is exactly the pivot's SCC.
+
+// The first blocks's threads try one candidate each: it starts in both
+// directions if both searches may still reach it.  Its two items follow the
+// frontiers' (from `at`).  Returns the items' end (block 0 only; the other
+// blocks return `at`).  All threads of every block call it.
+__device__ __forceinline__ unsigned long long
+seed_start(fwbw_args const& a, unsigned long long* aw, unsigned long long at, fwbw_smem& sm)
+{
+  for (int i = blockIdx.x * R_THREADS + threadIdx.x; i < LINK_WORDS - 8; i += gridDim.x * R_THREADS) a.links[i] = 0;
+  if (blockIdx.x != 0) return at;
+  static_assert(R_THREADS == 256, "a thread per label");
+  uint32_t const t  = threadIdx.x;
+  uint32_t       v  = 0;
+  bool           ok = t > 0 && t <= a.seeds; // label 0 is the pivot's
+  if (ok) {
+    v  = a.seed_ids[static_cast<uint64_t>(t - 1) * a.seed_n / a.seeds];
+    ok = v < a.n && ((__ldcg(a.cand + (v >> 5)) >> (v & 31)) & (__ldcg(a.cand_bw + (v >> 5)) >> (v & 31)) & 1u) && bit_take(a.cand, v);
+  }
+  if (ok) {
+    // (a candidate listed twice is taken once)
+    bit_take(a.cand_bw, v);
+    bit_claim(a.vis_a, v);
+    bit_claim(a.vis_b, v);
+  }
+  unsigned const bal = __ballot_sync(0xFFFFFFFFu, ok);
+  if ((t & 31u) == 0) a.links[LINK_WORDS - 8 + t / 32] = bal | (t == 0 ? 1u : 0u); // labels in use
+  a.links[LINK_VERTEX + t] = ok ? v : UNDECIDED;
+  uint64_t       tot;
+  uint64_t const r = block_exclusive_scan<uint64_t, R_THREADS>(ok ? 1u : 0u, &tot);
+  if (ok) {
+    unsigned long long const item = AW_TAG | AW_TAKEN | static_cast<unsigned long long>(t) << 54 | v;
+    __stcg(aw + at + 2 * r, item);
+    __stcg(aw + at + 2 * r + 1, item | AW_BW);
+  }
+  (void)sm;
+  return at + 2 * tot;
+}
+
+// Lane l's 16 vertices [v0, v0 + 16) of a 512-vertex stretch: the bits of C
+// (both sets) and their labels.
+__device__ __forceinline__ uint32_t
+seed_stretch(fwbw_args const& a, uint64_t v0, uint4& f, uint4& b)
+{
+  uint32_t const w = static_cast<uint32_t>(v0 >> 5);
+  uint32_t const c = v0 < a.n ? ((__ldcg(a.vis_a + w) & __ldcg(a.vis_b + w)) >> (v0 & 31)) & 0xFFFFu : 0u;
+  f = b = make_uint4(0, 0, 0, 0);
+  if (c) f = __ldcg(reinterpret_cast<uint4 const*>(a.label + v0)), b = __ldcg(reinterpret_cast<uint4 const*>(a.label + a.label_n + v0));
+  return c;
+}
+__device__ __forceinline__ uint32_t
+seed_label(uint4 const& x, int i)
+{
+  uint32_t const w = i < 4 ? x.x : (i < 8 ? x.y : (i < 12 ? x.z : x.w));
+  return (w >> (8 * (i & 3))) & 255u;
+}
+
+// The links between start vertices, then the ones that the pivot
+// reaches by them into good[0..8) and the ones that reach it into good[8..16)
+// (shared memory).  1: all in use are in both; 0: not; -1: a barrier gave up.
+// All threads of every block call it.
+__device__ __forceinline__ int
+seed_links(fwbw_args const& a, uint32_t* mat /* 2048 words of shared memory */, uint32_t* good, unsigned long long& epoch)
+{
+  __shared__ uint32_t s_fw[8], s_bw[8];
+  uint32_t const      t = threadIdx.x;
+  for (uint32_t i = t; i < 2048; i += R_THREADS) mat[i] = 0;
+  __syncthreads();
+  for (uint64_t v0 = (static_cast<uint64_t>(blockIdx.x) * R_THREADS + t) * 16; v0 < a.n; v0 += static_cast<uint64_t>(gridDim.x) * R_THREADS * 16) {
+    uint4          f, b;
+    uint32_t const c = seed_stretch(a, v0, f, b);
+    if (!c) continue;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      uint32_t const x = seed_label(f, i), y = seed_label(b, i);
+      if (((c >> i) & 1u) && x != y && !((mat[x * 8 + y / 32] >> (y & 31)) & 1u)) atomicOr(mat + x * 8 + y / 32, 1u << (y & 31));
+    }
+  }
+  // a start vertex whose neighbours were all reached from others has no other
+  // vertex of its label: its own rows give its links (i reaches j when an
+  // out-neighbour reaches j, h reaches i when h reaches an in-neighbour)
+  unsigned const lane = t & 31u;
+  for (uint32_t l = blockIdx.x * (R_THREADS / 32) + t / 32; l < 256; l += gridDim.x * (R_THREADS / 32)) {
+    uint32_t const v = __ldcg(a.links + LINK_VERTEX + l);
+    if (v >= a.n) continue;
+#pragma unroll 1
+    for (int dir = 0; dir < 2; ++dir) {
+      uint64_t const* head = dir ? a.bh : a.fh;
+      uint32_t const* adj  = dir ? a.bc : a.fc;
+      uint32_t const* set  = dir ? a.vis_a : a.vis_b;
+      uint64_t const  e    = head[v + 1] - head[v] > HEAVY_ROW ? head[v] + HEAVY_ROW : head[v + 1];
+      for (uint64_t x = head[v] + lane; x < e; x += 32) {
+        uint32_t const w = adj[x];
+        if (!((__ldcg(set + (w >> 5)) >> (w & 31)) & 1u)) continue;
+        uint32_t const o    = __ldcg(a.label + (dir ? 0 : a.label_n) + w);
+        uint32_t const from = dir ? o : l, to = dir ? l : o;
+        if (from != to) atomicOr(mat + from * 8 + to / 32, 1u << (to & 31));
+      }
+    }
+  }
+  __syncthreads();
+  for (uint32_t i = t; i < 2048; i += R_THREADS)
+    if (mat[i] && (mat[i] & ~__ldcg(a.links + i))) atomicOr(a.links + i, mat[i]);
+  if (!gsync(a, epoch)) return -1;
+  for (uint32_t i = t; i < 2048; i += R_THREADS) mat[i] = __ldcg(a.links + i);
+  if (t < 8) s_fw[t] = s_bw[t] = t == 0 ? 1u : 0u;
+  __syncthreads();
+  // thread t: start vertex t; both closures from the pivot's label, until
+  // neither grows
+  for (bool grew = true; grew;) {
+    bool more = false;
+    bool const inf = (s_fw[t / 32] >> (t & 31)) & 1u, inb = (s_bw[t / 32] >> (t & 31)) & 1u;
+    bool       hit = false;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      uint32_t const row = mat[t * 8 + k];
+      if (inf && (row & ~s_fw[k])) atomicOr(s_fw + k, row), more = true;
+      hit |= (row & s_bw[k]) != 0;
+    }
+    if (hit && !inb) atomicOr(s_bw + t / 32, 1u << (t & 31)), more = true;
+    grew = __syncthreads_or(more);
+  }
+  uint32_t const used = t < 8 ? __ldcg(a.links + LINK_WORDS - 8 + t) : 0u;
+  if (t < 8) good[t] = s_fw[t], good[8 + t] = s_bw[t];
+  return __syncthreads_or(t < 8 && (used & ~(s_fw[t] & s_bw[t]))) ? 0 : 1;
+}
+
+// Both searches start again inside C: reached = C's vertices with a good
+// label, candidates = the others of C.
+__device__ __forceinline__ void
+seed_restart(fwbw_args const& a, uint32_t const* good)
+{
+  unsigned const lane = threadIdx.x & 31u;
+  uint64_t const span = (static_cast<uint64_t>(a.n) + 511) & ~511ull;
+  for (uint64_t v0 = (static_cast<uint64_t>(blockIdx.x) * R_THREADS + threadIdx.x) * 16; v0 < span; v0 += static_cast<uint64_t>(gridDim.x) * R_THREADS * 16) {
+    uint4          f, b;
+    uint32_t const c  = seed_stretch(a, v0, f, b);
+    uint32_t       mf = 0, mb = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      uint32_t const x = seed_label(f, i), y = seed_label(b, i);
+      mf |= ((good[x / 32] >> (x & 31)) & 1u) << i;
+      mb |= ((good[8 + y / 32] >> (y & 31)) & 1u) << i;
+    }
+    // two lanes share a bitmap word: the even one writes it
+    uint32_t const c2 = c | __shfl_down_sync(0xFFFFFFFFu, c, 1) << 16;
+    mf &= c, mb &= c;
+    uint32_t const f2 = mf | __shfl_down_sync(0xFFFFFFFFu, mf, 1) << 16, b2 = mb | __shfl_down_sync(0xFFFFFFFFu, mb, 1) << 16;
+    if (!(lane & 1u) && v0 < a.n) {
+      uint32_t const w = static_cast<uint32_t>(v0 >> 5);
+      a.vis_a[w]   = f2;
+      a.cand[w]    = c2 & ~f2;
+      a.vis_b[w]   = b2;
+      a.cand_bw[w] = c2 & ~b2;
+    }
+  }
+}
 
 // Runs the rest of the search from frontier fq0[0, qn0) (direction d0).
 // With d1 (a joint phase) the other search runs in the same phase from its
@@ -1085,7 +1286,7 @@ struct aw_sink
 // nothing is left anywhere.
 __device__ __forceinline__ int
 run_async(fwbw_args const& a, uint32_t const* fq0, uint32_t qn0, aw_dir const d0, uint32_t const* fq1, uint32_t qn1, aw_dir const* d1, unsigned long long& epoch,
-          uint64_t& edges, fwbw_smem& sm)
+          uint64_t& edges, fwbw_smem& sm, bool seeded)
 {
   unsigned long long* const aw   = a.aw;
   unsigned long long* const head = a.aq;
@@ -1099,9 +1300,17 @@ run_async(fwbw_args const& a, uint32_t const* fq0, uint32_t qn0, aw_dir const d0
   uint32_t const            qb    = joint ? qn1 : 0u;
   for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * R_THREADS + threadIdx.x; i < qn0 + qb; i += static_cast<uint64_t>(gridDim.x) * R_THREADS)
     __stcg(aw + i, i < qn0 ? AW_TAG | AW_TAKEN | __ldcg(fq0 + i) : AW_TAG | AW_TAKEN | AW_BW | __ldcg(fq1 + (i - qn0)));
-  if (blockIdx.x == 0 && threadIdx.x == 0) *head = 0, *tail = qn0 + qb, *done = 0;
+  unsigned long long first = qn0 + qb;
+  if (seeded) {
+    first = seed_start(a, aw, first, sm);
+    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * R_THREADS + threadIdx.x; i < 2 * a.label_n / 16; i += static_cast<uint64_t>(gridDim.x) * R_THREADS)
+      __stcg(reinterpret_cast<uint4*>(a.label) + i, make_uint4(0, 0, 0, 0)); // everything reached so far: the pivot's
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *head = 0, *tail = first, *done = 0;
   if (!gsync(a, epoch)) return SEARCH_FAILED;
-  aw_sink const sink{ reinterpret_cast<unsigned long long*>(&sm.warp[threadIdx.x >> 5]), aw, tail, cap };
+  unsigned long long const keep = seeded ? AW_BW | AW_LABEL : AW_BW; // what an item's finds inherit
+  uint32_t const           smask = seeded ? 0x1FFFFFu : 0x1FFFFFFFu;
+  aw_sink const sink{ reinterpret_cast<unsigned long long*>(&sm.warp[threadIdx.x >> 5]), aw, tail, cap, seeded ? min(max(a.n / AW_KEEP_SPAN, AW_KEEP_MIN), AW_KEEP_MAX) : AW_LOCAL_KEEP };
   bool          failed      = false;
   uint32_t      unpublished = 0; // worklist items this warp finished, not yet added to done
   uint32_t      ls_n        = 0; // items on this warp's stack (warp-uniform)
@@ -1162,9 +1371,9 @@ run_async(fwbw_args const& a, uint32_t const* fq0, uint32_t qn0, aw_dir const d0
     unsigned const gmask = __ballot_sync(0xFFFFFFFFu, got);
     if (gmask) {
       uint32_t const           v   = static_cast<uint32_t>(item);
-      uint32_t const           sl  = static_cast<uint32_t>(item >> 33) & 0x1FFFFFFFu;
-      unsigned long long const dir = item & AW_BW;
-      aw_dir const             d   = dir ? e1 : d0;
+      uint32_t const           sl  = static_cast<uint32_t>(item >> 33) & smask;
+      unsigned long long const dir = item & keep;
+      aw_dir const             d   = dir & AW_BW ? e1 : d0;
       uint64_t                 b = 0, e = 0;
       bool                     won = got;
       if (got) {
@@ -1173,6 +1382,7 @@ run_async(fwbw_args const& a, uint32_t const* fq0, uint32_t qn0, aw_dir const d0
         if (!(item & AW_TAKEN) && sl == 0) won = bit_take(d.avail, v);
         b = d.head[v], e = d.head[v + 1];
         if (!(item & AW_TAKEN) && sl == 0 && won) bit_set_async(d.mark, v);
+        if (seeded && sl == 0 && won) a.label[(dir & AW_BW ? a.label_n : 0) + v] = static_cast<uint8_t>(dir >> 54);
         if (!won) e = b;
       }
       if (got && e - b > HEAVY_ROW) {
@@ -1230,7 +1440,7 @@ run_async(fwbw_args const& a, uint32_t const* fq0, uint32_t qn0, aw_dir const d0
         unsigned const           l   = __ffs(todo) - 1;
         uint64_t const           b0  = __shfl_sync(0xFFFFFFFFu, b, l), e0 = __shfl_sync(0xFFFFFFFFu, e, l);
         unsigned long long const dl  = __shfl_sync(0xFFFFFFFFu, dir, l);
-        aw_dir const             dd_ = dl ? e1 : d0;
+        aw_dir const             dd_ = dl & AW_BW ? e1 : d0;
         for (uint64_t xb = b0; xb < e0; xb += 32) {
           uint64_t const x1 = xb + lane;
           uint32_t       w  = 0;
@@ -1362,9 +1572,20 @@ struct jctl
   uint32_t           restrict_to[2]; // 1: cut this search's candidates down to the other's set first
   uint32_t           capped, async, any_td, any_bu;
   uint32_t           cw;          // words per bottom-up chunk (bu_chunk_words)
+  uint32_t           seeded;      // a worklist phase with several start vertices has run
   uint32_t           cnt[2];
 };
 __shared__ jctl s_j;
+
+// Do the two searches together grow slowly?  Reached ~ levels^k has a
+// frontier of k / levels of it, so k <= 3: a line, a plane, a space -- not a
+// random graph, whose frontier grows by a factor per level (1.6 and more
+// fails at 8 levels) and ends soon anyway.
+__device__ __forceinline__ bool
+joint_slow(unsigned long long qmask)
+{
+  return ((s_j.c[0] & qmask) + (s_j.c[1] & qmask)) * max(s_j.lvl[0], s_j.lvl[1]) <= 3 * (s_j.seen[0] + s_j.seen[1]);
+}
 
 // The level loop's control where a launch handed off its worklist phase
 // (written by block 0, read by every block of the resume launch).
@@ -1400,7 +1621,7 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
       s_j.live[d]                                                      = 1;
       s_j.restrict_to[d]                                               = 0;
     }
-    if (!resume) s_j.capped = 0;
+    if (!resume) s_j.capped = 0, s_j.seeded = 0;
   }
   int  rc         = SEARCH_DONE;
   bool resume_now = resume; // the first iteration of a resume launch starts at its worklist phase
@@ -1462,7 +1683,10 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
           else if (s_j.mode[d] == 0 && mf * a.alpha > s_j.m_u[d]) s_j.mode[d] = 1;
           s_j.kind[d] = s_j.mode[d] ? JK_BU : JK_TD;
           s_j.grp[d]  = s_j.mode[d] && s_j.cw == 32 ? bu_group_size(n_und > s_j.seen[d] ? n_und - s_j.seen[d] : 0, a.n) : 1u;
-          if (!(s_j.mode[d] == 0 && s_j.lvl[d] >= ASYNC_AFTER && qn <= ASYNC_FRONTIER)) async = false;
+          if (!(s_j.mode[d] == 0 && s_j.lvl[d] >= ASYNC_SLOW && qn <= ASYNC_FRONTIER)) async = false;
+          // early only with a frontier as of a plane: a few vertices wide it may
+          // be a path into a dense part, which levels expand faster
+          if (s_j.lvl[d] < ASYNC_AFTER && !(joint_slow(qmask) && (s_j.c[0] & qmask) + (s_j.c[1] & qmask) >= s_j.lvl[d])) async = false;
         }
         s_j.async  = async && live && !s_j.capped;
         s_j.any_td = s_j.kind[0] == JK_TD || s_j.kind[1] == JK_TD;
@@ -1486,7 +1710,7 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
         }
     }
     resume_now = false;
-    if (MINB != 2 && s_j.async) {
+    if (MINB != 3 && s_j.async) {
       // the worklist phase runs in a launch with more registers per thread
       // (its hop chains stay in flight without spills): save the control
       // and end this launch; the resume launch starts at this point
@@ -1500,7 +1724,7 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
       }
       return SEARCH_HANDOFF;
     }
-    if constexpr (MINB == 2) {
+    if constexpr (MINB == 3) {
       if (s_j.async) {
         // long and thin: both searches finish on the worklist
         uint64_t   ea = 0;
@@ -1511,13 +1735,34 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
         aw_dir const w1{ D1.td_head, D1.td_adj, D1.avail, D1.mark };
         frontier_buf const f0 = s_j.lvl[d0] == 0 ? a.seed : jbuf(D0, glvl);
         frontier_buf const f1 = s_j.lvl[1] == 0 ? a.seed : jbuf(D1, glvl);
-        int const r = run_async(a, f0.q, static_cast<uint32_t>(s_j.c[d0] & qmask), w0, f1.q, static_cast<uint32_t>(s_j.c[1] & qmask), two ? &w1 : nullptr, epoch, ea, sm);
+        // several start vertices where the searches grow slowly and most of the
+        // graph is undecided (near the giant-component threshold of a random
+        // graph, mean degree below 1.7, less than 2/3 are and most candidates
+        // lie outside the SCC: a restart for nothing); block-uniform
+        bool const seeded = two && a.seeds && !s_j.seeded && static_cast<uint64_t>(n_und) * 3 >= static_cast<uint64_t>(a.n) * 2 && joint_slow(qmask);
+        int const r = run_async(a, f0.q, static_cast<uint32_t>(s_j.c[d0] & qmask), w0, f1.q, static_cast<uint32_t>(s_j.c[1] & qmask), two ? &w1 : nullptr, epoch, ea, sm, seeded);
         if (r != SEARCH_DONE) return r;
         stamp(a, 13);
+        int exact = 1;
+        if (seeded) {
+          uint32_t* const mat  = reinterpret_cast<uint32_t*>(sm.warp);
+          uint32_t* const good = mat + 2048;
+          exact                = seed_links(a, mat, good, epoch);
+          if (exact < 0) return SEARCH_FAILED;
+          if (!exact) {
+            seed_restart(a, good);
+            if (!gsync(a, epoch)) return SEARCH_FAILED;
+          }
+          stamp(a, 17);
+        }
         if (threadIdx.x == 0) {
           s_j.edges_td[d0] += ea;
           for (int d = 0; d < 2; ++d)
-            if (s_j.live[d]) s_j.c[d] = 0, s_j.mode[d] = 0, s_j.mat[d] = 0, s_j.lvl[d] += 1; // nothing queued: next it runs dry (or fixes up cut rows)
+            if (s_j.live[d]) {
+              s_j.c[d] = 0, s_j.mode[d] = 0, s_j.mat[d] = 0, s_j.lvl[d] += 1; // nothing queued: next it runs dry (or fixes up cut rows)
+              if (!exact) s_j.c[d] = 1, s_j.mode[d] = 1, s_j.seen[d] = 1;     // the restarted sets: next a bottom-up sweep
+            }
+          s_j.seeded |= seeded ? 1u : 0u;
         }
         if (tally) st->async_phases += 1;
         continue;
@@ -2086,7 +2331,7 @@ run_trim(fwbw_args const& a, uint32_t& glvl, unsigned long long& epoch)
       rc = SEARCH_CAPPED;
       break;
     }
-    if (lvl >= ASYNC_AFTER && qn <= ASYNC_FRONTIER && a.aw && !first && __ldcg(&st->hq_n[2 * (glvl % 3)]) == 0 && __ldcg(&st->hq_n[2 * (glvl % 3) + 1]) == 0) {
+    if (lvl >= ASYNC_SLOW && qn <= ASYNC_FRONTIER && a.aw && !first && __ldcg(&st->hq_n[2 * (glvl % 3)]) == 0 && __ldcg(&st->hq_n[2 * (glvl % 3) + 1]) == 0) {
       // long and thin: the rest of the fixpoint on the worklist (no heavy
       // rows are pending from the level before)
       rc = run_trim_async(a, a.fb[glvl & 1].q, static_cast<uint32_t>(qn), epoch, dec, edges);
@@ -2146,8 +2391,10 @@ write_ids(fwbw_args const& a, uint32_t words, bool search, uint32_t scc)
 
 // MINB: blocks per SM the launch is compiled for.  The level loop runs
 // with 4 (64 registers per thread); a search that moves to the worklist
-// phase hands off to a resume launch with 2 (128 registers), whose hop
-// chains keep their loads in flight without spills.
+// phase hands off to a resume launch with 3 (80 registers), whose hop chains
+// keep their loads in flight without spills: with several start vertices
+// the phase has work for every warp (RGG 2^24, whole call: 2 blocks 6.44 ms,
+// 3: 5.73, 4: 5.37 but slower on shorter phases).
 template<int MINB>
 __global__ void __launch_bounds__(R_THREADS, MINB)
 k_fwbw(fwbw_args a)
@@ -2501,7 +2748,7 @@ resume_grid(kspn_context* ctx)
 {
   if (!ctx->resume_grid) {
     int bps = 0, sms = 0;
-    KSPN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_fwbw<2>, R_THREADS, 0));
+    KSPN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_fwbw<3>, R_THREADS, 0));
     KSPN_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     if (bps < 1) throw error{ KSPN_ERR_CUDA, "persistent FW-BW resume kernel does not fit on an SM" };
     ctx->resume_grid = static_cast<unsigned>(std::min<int>(bps * sms, AW_GRID_MAX));
@@ -2594,6 +2841,14 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
   a.gate         = gated ? ws.ctr + CTR_ERR : nullptr;
   a.jsave        = static_cast<char*>(ws.gbar) + 2048;
   a.resume       = 0;
+  // start vertices for a worklist phase: one per SEED_SPAN vertices (a hop
+  // costs the same for one or hundreds of searches in flight)
+  a.seeds        = g.m < (1ull << 31) ? std::min<uint32_t>(255, g.n / SEED_SPAN) : 0u;
+  a.seed_n       = pivot_candidates(g.n);
+  a.seed_ids     = reinterpret_cast<uint32_t const*>(ws.pivot + 4096);
+  a.label        = reinterpret_cast<uint8_t*>(ws.label);
+  a.label_n      = (static_cast<uint64_t>(g.n) + 15) & ~15ull;
+  a.links        = ws.links;
   static_assert(sizeof(fwbw_args) <= sizeof(ctx->fwbw_last), "launch arguments must fit their copy in the context");
   static_assert(sizeof(joint_save) <= 2048, "saved level control must fit its workspace slot");
   std::memcpy(ctx->fwbw_last, &a, sizeof(a));
@@ -2611,7 +2866,7 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
 }
 
 // After the stream was synchronised: a launch that handed off its worklist
-// phase is continued by the resume launch (same arguments, 128 registers
+// phase is continued by the resume launch (same arguments, 80 registers
 // per thread; one more host round trip, only on graphs that reach that
 // phase); then barrier failures and level caps.  Returns whether a resume
 // launch ran.
@@ -2627,7 +2882,7 @@ check_persistent(kspn_context* ctx)
     a.resume     = 1;
     void* args[] = { &a };
     barrier_for_grid(ctx, resume_grid(ctx));
-    KSPN_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(&k_fwbw<2>), dim3(resume_grid(ctx)), dim3(R_THREADS), args, 0, ctx->stream));
+    KSPN_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(&k_fwbw<3>), dim3(resume_grid(ctx)), dim3(R_THREADS), args, 0, ctx->stream));
     ctx->launches += 1;
     if (ctx->fwbw_after) KSPN_CUDA(cudaEventRecord(ctx->fwbw_after, ctx->stream));
     KSPN_CUDA(cudaMemcpyAsync(hs, ctx->ws.rstate, sizeof(reach_state), cudaMemcpyDeviceToHost, ctx->stream));
