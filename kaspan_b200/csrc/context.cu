@@ -321,7 +321,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
       if (decided < g.n) fwbw_from(pivot);
       if (decided < g.n) add(KSPN_PHASE_TRIM_NORMAL, trim_1_normal(ctx, g, und, scc_id));
       if (decided < g.n) add(KSPN_PHASE_TRIM_NORMAL, trim_1_normal(ctx, g, und, scc_id));
-      if (decided < g.n) add(KSPN_PHASE_RESIDUAL, residual(ctx, g, und, scc_id, nullptr));
+      if (decided < g.n) add(KSPN_PHASE_RESIDUAL, residual(ctx, g, und, scc_id, nullptr, g.n - decided));
       label_rounds(false);
       break;
     case KSPN_PIPELINE_TRIM_EX: // scc_trim_ex.hpp:33-99
@@ -331,11 +331,11 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
       break;
     case KSPN_PIPELINE_TRIM_EX_LIGHT_RESIDUAL: // scc_trim_ex_light_residual.hpp:33-118 (threshold 0 at one rank)
       if (decided < g.n) add(KSPN_PHASE_TRIM, trim_fixpoint(ctx, g, und, scc_id, false, 0));
-      if (decided < g.n) add(KSPN_PHASE_RESIDUAL, residual(ctx, g, und, scc_id, nullptr));
+      if (decided < g.n) add(KSPN_PHASE_RESIDUAL, residual(ctx, g, und, scc_id, nullptr, g.n - decided));
       label_rounds(false);
       break;
     default: // KSPN_PIPELINE_TRIM_EX_RESIDUAL, scc_trim_ex_residual.hpp:33-127 (threshold 0 at one rank)
-      if (decided < g.n) add(KSPN_PHASE_RESIDUAL, residual(ctx, g, und, scc_id, nullptr));
+      if (decided < g.n) add(KSPN_PHASE_RESIDUAL, residual(ctx, g, und, scc_id, nullptr, g.n - decided));
       label_rounds(false);
       break;
     }
@@ -429,7 +429,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
       if (decided < g.n) fwbw_again();
       // what is left splits into small pieces on most graphs: Tarjan per
       // piece in shared memory; larger pieces go on to the rounds below
-      if (decided < g.n) add(KSPN_PHASE_RESIDUAL, residual(ctx, g, und, scc_id, nullptr));
+      if (decided < g.n) add(KSPN_PHASE_RESIDUAL, residual(ctx, g, und, scc_id, nullptr, g.n - decided));
     } else {
       uint32_t pivot = trim_1_first(ctx, g, und, scc_id, nullptr, nullptr, false);
       add(KSPN_PHASE_TRIM_FIRST, ctx->h_ctr[CTR_AUX]);
@@ -467,8 +467,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
     }
     if (st) st->rounds = rounds;
   }
-  if (decided != g.n || (!und_checked && count_undecided(ctx, g.n, und) != 0)) throw error{ KSPN_ERR_INTERNAL, "decided-vertex count does not match n" };
-  if (st) st->edges_scanned = ctx->h_ctr64[0] + ctx->td_edges;
+  if (decided != g.n) throw error{ KSPN_ERR_INTERNAL, "decided-vertex count does not match n" };
   // trim (id = itself), trim-2 (id = the smaller of the pair) and FW-BW
   // (id = smallest member) already name components canonically; label
   // searches name them after their root, so only then is a relabel needed
@@ -477,11 +476,17 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
     // event (now ev[0]) the host already waited for: no further sync
     t_end = ctx->ev[0];
   } else {
+    // und is counted on the way: the count comes back with the relabel's
+    // check, or alone
+    count_undecided_async(ctx, g.n, und);
     if (label_ran) canonicalise(ctx, g.n, scc_id, ws.label, true);
-    add(KSPN_PHASE_CANON, 0);
     KSPN_CUDA(cudaEventRecord(t_end, ctx->stream));
+    if (!label_ran) read_counters(ctx);
+    if (ctx->h_ctr[CTR_LEFT]) throw error{ KSPN_ERR_INTERNAL, "decided-vertex count does not match n" };
+    add(KSPN_PHASE_CANON, 0);
     KSPN_CUDA(cudaEventSynchronize(t_end));
   }
+  if (st) st->edges_scanned = ctx->h_ctr64[0] + ctx->td_edges;
   if (st) {
     float ms = 0;
     KSPN_CUDA(cudaEventElapsedTime(&ms, t_begin, t_end));
@@ -1082,7 +1087,7 @@ kspn_residual(kspn_context* ctx, uint32_t n, uint64_t m, const uint64_t* d_fw_he
     ensure_workspace(ctx, n, m);
     dgraph const   g{ n, m, d_fw_head, d_fw_csr, nullptr, nullptr };
     uint32_t       left = 0;
-    uint32_t const d    = n ? residual(ctx, g, reinterpret_cast<uint32_t*>(d_undecided), d_scc_id, &left) : 0;
+    uint32_t const d    = n ? residual(ctx, g, reinterpret_cast<uint32_t*>(d_undecided), d_scc_id, &left, n) : 0;
     if (decided) *decided = d;
     if (pieces_left) *pieces_left = left;
   });

@@ -275,6 +275,7 @@ enum ctr_slot : int
   CTR_COUNT = 16, // slots 5.. are phase-specific (8: expansion tile count)
   CTR_RES_HEAVY  = 5, // residual: heavy rows listed by k_res_hook
   CTR_TRIM_HEAVY = 6, // trim push levels (host-driven): heavy out-rows at 6, in-rows at 7; live counts: 9
+  CTR_LEFT      = 10, // undecided vertices at a pipeline's end (count_undecided_async)
   CTR_PV_TICKET = 15 // trim_1_first: blocks finished (the last one reduces the pivot)
 };
 
@@ -527,8 +528,8 @@ void mlp_adam(kspn_context* ctx, float* params, float const* grad, float* m, flo
 void learned_pivot(kspn_context* ctx, dgraph const& g, float const* params, bool check = true);
 // residual.cu: Tarjan per weakly connected undecided piece that fits a warp's
 // shared memory; returns vertices decided, *pieces_left = pieces left over
-uint32_t residual(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t* pieces_left);
-uint32_t count_undecided(kspn_context* ctx, uint32_t n, uint32_t const* und);
+uint32_t residual(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t* pieces_left, uint64_t undecided);
+void     count_undecided_async(kspn_context* ctx, uint32_t n, uint32_t const* und); // into ws.ctr[CTR_LEFT]
 
 // reach.cu
 size_t reach_state_bytes();

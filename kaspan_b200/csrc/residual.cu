@@ -8,24 +8,30 @@
 // named by its smallest original vertex id.
 //
 // On the device the sub-graph splits into weakly connected pieces (an SCC
-// never spans two), and one warp decomposes each small piece in shared
-// memory:
-//   1. union-find over the undecided vertices' out-edges to undecided
-//      vertices (hooking the larger root under the smaller with atomicCAS,
-//      path halving), then every entry set to its root by a pass in which
-//      only v's own thread writes parent[v]; every loop bounded;
-//   2. the undecided vertices in id order (ordered compaction), stably
-//      radix-sorted by root: each piece is a segment, ascending inside;
-//   3. a warp per segment of at most RS_MAXV vertices and RS_MAXE internal
-//      edges builds the piece's CSR in shared memory (local ids by binary
-//      search in the sorted segment), lane 0 runs an iterative Tarjan with
-//      explicit stacks, and the warp writes each member's SCC id (its
-//      smallest member: the smallest local index, since the segment is
-//      ascending) and clears it from und.
+// never spans two), and one warp decomposes each small piece:
+//   1. the undecided vertices are listed (every later pass runs over the
+//      list), and union-find over their out-edges to undecided vertices joins
+//      them (hooking the larger root under the smaller with atomicCAS, path
+//      halving); then every entry is set to its root by a pass in which only
+//      v's own thread writes parent[v]; every loop bounded;
+//   2. in that pass each vertex takes a place in its piece (an atomic count at
+//      the root); a pass over the roots gives each piece a range of one member
+//      array, and each vertex enters its place;
+//   3. a piece of up to 32 vertices goes to a warp, lane = vertex: rows become
+//      bit masks, Warshall's closure takes one shuffle per vertex, and an SCC is
+//      the closure and its transpose (one ballot per vertex); a piece of up to
+//      RS_MAXV vertices and RS_MAXE internal edges goes to a warp's
+//      shared-memory Tarjan (lane 0, explicit stacks).  Either way each member
+//      gets its SCC's smallest vertex and leaves und.
 // Larger pieces stay undecided; the pipeline's label rounds finish them.
+// Bound: launches and the latency of a few dependent loads each.  RGG of 10^6
+// vertices (29,636 undecided, whole step): 390 us with ordered compaction,
+// a radix sort by root and every piece through Tarjan.
 #include "kspn_internal.cuh"
 #include "prim.cuh"
 #include "tarjan_smem.cuh"
+
+#include <algorithm>
 
 namespace kspn {
 
@@ -62,11 +68,35 @@ rs_find(uint32_t* parent, uint32_t x)
   return UNDECIDED;
 }
 
+// The undecided vertices (in no particular order), each a root of its own
+// with an empty piece.
 __global__ void __launch_bounds__(RS_THREADS)
-k_res_init(uint32_t n, uint32_t const* __restrict__ und, uint32_t* __restrict__ parent)
+k_res_list(uint32_t n, uint32_t const* __restrict__ und, uint32_t* __restrict__ parent, uint32_t* __restrict__ count, uint32_t* __restrict__ list, uint32_t* list_n)
 {
-  for (uint64_t v = static_cast<uint64_t>(blockIdx.x) * RS_THREADS + threadIdx.x; v < n; v += static_cast<uint64_t>(gridDim.x) * RS_THREADS)
-    if (und_has(und, static_cast<uint32_t>(v))) parent[v] = static_cast<uint32_t>(v);
+  unsigned const lane  = threadIdx.x & 31u;
+  uint32_t const words = (n + 31) / 32, span = (words + 31) & ~31u;
+  for (uint32_t w = blockIdx.x * RS_THREADS + threadIdx.x; w < span; w += gridDim.x * RS_THREADS) {
+    uint32_t x = w < words ? und[w] : 0u;
+    if (w == words - 1 && (n & 31)) x &= (1u << (n & 31)) - 1u;
+    uint32_t const c    = __popc(x);
+    uint32_t       incl = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      uint32_t const y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= static_cast<unsigned>(d)) incl += y;
+    }
+    uint32_t const tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    if (!tot) continue; // warp-uniform
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(list_n, tot);
+    at = __shfl_sync(0xFFFFFFFFu, at, 0) + incl - c;
+    for (; x; x &= x - 1) {
+      uint32_t const v = w * 32 + __ffs(x) - 1;
+      list[at++]       = v;
+      parent[v]        = v;
+      count[v]         = 0;
+    }
+  }
 }
 
 // u ~ v (both undecided); false when a loop bound was reached
@@ -99,13 +129,14 @@ rs_edge(uint32_t const* und, uint32_t* parent, uint32_t* err, uint32_t u, uint32
 // up to 32 edges, the warp one of up to HEAVY_ROW; longer rows are listed
 // for k_res_hook_heavy.
 __global__ void __launch_bounds__(RS_THREADS)
-k_res_hook(uint32_t n, uint32_t const* __restrict__ und, uint64_t const* __restrict__ fh, uint32_t const* __restrict__ fc, uint32_t* parent, uint32_t* err, uint32_t* heavy, uint32_t* heavy_n)
+k_res_hook(uint32_t const* __restrict__ list, uint32_t const* __restrict__ list_n, uint32_t const* __restrict__ und, uint64_t const* __restrict__ fh, uint32_t const* __restrict__ fc,
+           uint32_t* parent, uint32_t* err, uint32_t* heavy, uint32_t* heavy_n)
 {
   unsigned const lane = threadIdx.x & 31u;
-  uint64_t const span = (static_cast<uint64_t>(n) + 31) & ~31ull;
-  for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * RS_THREADS + threadIdx.x; t < span; t += static_cast<uint64_t>(gridDim.x) * RS_THREADS) {
-    uint32_t const u    = static_cast<uint32_t>(t);
-    bool const     have = t < n && und_has(und, u);
+  uint32_t const k    = *list_n;
+  for (uint32_t t0 = blockIdx.x * RS_THREADS + (threadIdx.x & ~31u); t0 < k; t0 += gridDim.x * RS_THREADS) {
+    bool const     have = t0 + lane < k;
+    uint32_t const u    = have ? list[t0 + lane] : 0u;
     uint64_t       b = 0, e = 0;
     if (have) b = fh[u], e = fh[u + 1];
     uint64_t const len = e - b;
@@ -131,29 +162,17 @@ k_res_hook_heavy(uint32_t const* __restrict__ und, uint64_t const* __restrict__ 
   });
 }
 
-// Shortens the trees (path halving; another thread's halving store may
-// overwrite a root written here with an older ancestor, so k_res_flatten
-// finishes the job).
-__global__ void __launch_bounds__(RS_THREADS)
-k_res_compress(uint32_t n, uint32_t const* __restrict__ und, uint32_t* parent, uint32_t* err)
-{
-  for (uint64_t v = static_cast<uint64_t>(blockIdx.x) * RS_THREADS + threadIdx.x; v < n; v += static_cast<uint64_t>(gridDim.x) * RS_THREADS) {
-    if (!und_has(und, static_cast<uint32_t>(v))) continue;
-    uint32_t const r = rs_find(parent, static_cast<uint32_t>(v));
-    if (r == UNDECIDED) atomicExch(err, 1u);
-    else parent[v] = r;
-  }
-}
-
 // parent[v] = root of v, each entry written only by v's own thread (the
-// walk itself writes nothing), so every entry ends at its root.
+// walk itself writes nothing), so every entry ends at its root; and v's
+// place in its piece.
 __global__ void __launch_bounds__(RS_THREADS)
-k_res_flatten(uint32_t n, uint32_t const* __restrict__ und, uint32_t* parent, uint32_t* err)
+k_res_flatten(uint32_t const* __restrict__ list, uint32_t const* __restrict__ list_n, uint32_t* parent, uint32_t* count, uint32_t* __restrict__ place, uint32_t* err)
 {
-  for (uint64_t v = static_cast<uint64_t>(blockIdx.x) * RS_THREADS + threadIdx.x; v < n; v += static_cast<uint64_t>(gridDim.x) * RS_THREADS) {
-    if (!und_has(und, static_cast<uint32_t>(v))) continue;
-    uint32_t x  = static_cast<uint32_t>(v);
-    bool     ok = false;
+  uint32_t const k = *list_n;
+  for (uint32_t i = blockIdx.x * RS_THREADS + threadIdx.x; i < k; i += gridDim.x * RS_THREADS) {
+    uint32_t const v = list[i];
+    uint32_t       x = v;
+    bool           ok = false;
     for (uint32_t it = 0; it < RS_FIND; ++it) {
       uint32_t const p = __ldcg(parent + x);
       if (p == x) {
@@ -163,79 +182,149 @@ k_res_flatten(uint32_t n, uint32_t const* __restrict__ und, uint32_t* parent, ui
       x = p;
     }
     if (!ok) atomicExch(err, 1u);
-    else parent[v] = x;
-  }
-}
-
-struct f_und_popc
-{
-  uint32_t const* und;
-  uint32_t        n;
-  __device__ uint32_t operator()(uint64_t w) const
-  {
-    uint32_t x = und[w];
-    if ((w + 1) * 32 > n) x &= (n & 31) ? (1u << (n & 31)) - 1u : 0xFFFFFFFFu;
-    return __popc(x);
-  }
-};
-
-// (root, vertex) of every undecided vertex, in vertex order
-__global__ void __launch_bounds__(RS_THREADS)
-k_res_list(uint32_t n, uint32_t const* __restrict__ und, uint32_t const* __restrict__ pos, uint32_t const* __restrict__ parent, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals)
-{
-  uint32_t const words = (n + 31) / 32;
-  for (uint64_t w = static_cast<uint64_t>(blockIdx.x) * RS_THREADS + threadIdx.x; w < words; w += static_cast<uint64_t>(gridDim.x) * RS_THREADS) {
-    uint32_t x = und[w];
-    if ((w + 1) * 32 > n) x &= (n & 31) ? (1u << (n & 31)) - 1u : 0xFFFFFFFFu;
-    uint32_t j = pos[w];
-    for (; x; x &= x - 1, ++j) {
-      uint32_t const v = static_cast<uint32_t>(w) * 32 + __ffs(x) - 1;
-      keys[j]          = parent[v];
-      vals[j]          = v;
+    else {
+      parent[v] = x;
+      place[v]  = atomicAdd(count + x, 1u);
     }
   }
 }
 
-struct f_seg_head
+// Device counters of the pieces.
+struct rs_counts
 {
-  uint32_t const* keys;
-  __device__ uint32_t operator()(uint64_t i) const { return i == 0 || keys[i] != keys[i - 1] ? 1u : 0u; }
+  uint32_t list_n;  // undecided vertices
+  uint32_t members; // handed-out places of the member array
+  uint32_t small, mid; // pieces of at most 32 and of at most RS_MAXV vertices
 };
 
+// Every piece's range of the member array, and its list: small pieces from
+// the front of `pieces`, the others from its end (an entry per vertex holds
+// both).  Pieces of more than RS_MAXV vertices get none.
 __global__ void __launch_bounds__(RS_THREADS)
-k_res_segments(uint64_t k, uint32_t const* __restrict__ keys, uint32_t const* __restrict__ spos, uint32_t* __restrict__ seg_start)
+k_res_ranges(uint32_t const* __restrict__ list, uint32_t const* __restrict__ parent, uint32_t const* __restrict__ count, uint32_t* __restrict__ start, uint32_t* __restrict__ pieces, uint32_t cap,
+             rs_counts* rc, uint32_t* big)
 {
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * RS_THREADS + threadIdx.x; i < k; i += static_cast<uint64_t>(gridDim.x) * RS_THREADS)
-    if (i == 0 || keys[i] != keys[i - 1]) seg_start[spos[i]] = static_cast<uint32_t>(i);
-  if (blockIdx.x == 0 && threadIdx.x == 0) seg_start[spos[k]] = static_cast<uint32_t>(k);
+  unsigned const lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  uint32_t const k    = rc->list_n;
+  for (uint32_t t0 = blockIdx.x * RS_THREADS + (threadIdx.x & ~31u); t0 < k; t0 += gridDim.x * RS_THREADS) {
+    uint32_t const v    = t0 + lane < k ? list[t0 + lane] : UNDECIDED;
+    bool const     root = v != UNDECIDED && parent[v] == v;
+    uint32_t const c    = root ? count[v] : 0u;
+    uint32_t const take = c <= RS_MAXV ? c : 0u;
+    if (root && c > RS_MAXV) start[v] = UNDECIDED, atomicAdd(big, 1u);
+    uint32_t incl = take;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      uint32_t const y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= static_cast<unsigned>(d)) incl += y;
+    }
+    unsigned const sm = __ballot_sync(0xFFFFFFFFu, take && take <= 32), md = __ballot_sync(0xFFFFFFFFu, take > 32);
+    uint32_t       m0 = 0, s0 = 0, d0 = 0;
+    if (lane == 31 && incl) m0 = atomicAdd(&rc->members, incl);
+    if (lane == 0 && sm) s0 = atomicAdd(&rc->small, static_cast<uint32_t>(__popc(sm)));
+    if (lane == 0 && md) d0 = atomicAdd(&rc->mid, static_cast<uint32_t>(__popc(md)));
+    m0 = __shfl_sync(0xFFFFFFFFu, m0, 31), s0 = __shfl_sync(0xFFFFFFFFu, s0, 0), d0 = __shfl_sync(0xFFFFFFFFu, d0, 0);
+    if (take) {
+      start[v] = m0 + incl - take;
+      if (take <= 32) pieces[s0 + __popc(sm & lt)] = v;
+      else pieces[cap - 1 - (d0 + __popc(md & lt))] = v;
+    }
+  }
 }
 
-// One warp per piece of at most RS_MAXV vertices and RS_MAXE internal edges.
+__global__ void __launch_bounds__(RS_THREADS)
+k_res_members(uint32_t const* __restrict__ list, uint32_t const* __restrict__ list_n, uint32_t const* __restrict__ parent, uint32_t const* __restrict__ start, uint32_t const* __restrict__ place,
+              uint32_t* __restrict__ members)
+{
+  uint32_t const k = *list_n;
+  for (uint32_t i = blockIdx.x * RS_THREADS + threadIdx.x; i < k; i += gridDim.x * RS_THREADS) {
+    uint32_t const v = list[i], b = start[parent[v]];
+    if (b != UNDECIDED) members[b + place[v]] = v;
+  }
+}
+
+// One warp per piece of at most 32 vertices, lane = place in the piece.
+// und_in is the undecided set as the step found it (a vertex decided here
+// still counts as its own piece's).
+__global__ void __launch_bounds__(RS_THREADS)
+k_res_small(rs_counts const* __restrict__ rc, uint32_t const* __restrict__ pieces, uint32_t const* __restrict__ count, uint32_t const* __restrict__ start, uint32_t const* __restrict__ place,
+            uint32_t const* __restrict__ parent, uint32_t const* __restrict__ members, uint64_t const* __restrict__ fh, uint32_t const* __restrict__ fc, uint32_t* und, uint32_t* __restrict__ scc_id,
+            uint32_t* decided, uint32_t* big)
+{
+  unsigned const lane = threadIdx.x & 31u;
+  uint32_t const P    = rc->small;
+  uint32_t       dec  = 0;
+  for (uint32_t p = blockIdx.x * (RS_THREADS / 32) + (threadIdx.x >> 5); p < P; p += gridDim.x * (RS_THREADS / 32)) {
+    uint32_t const root = pieces[p], k = count[root], b = start[root];
+    bool const     have = lane < k;
+    uint32_t const v    = have ? members[b + lane] : UNDECIDED;
+    uint64_t const e0   = have ? fh[v] : 0;
+    uint32_t const len  = have ? static_cast<uint32_t>(min(fh[v + 1] - e0, static_cast<uint64_t>(HEAVY_ROW) + 1)) : 0u;
+    bool           left = __any_sync(0xFFFFFFFFu, len > HEAVY_ROW); // a row too long for one lane: left to the later rounds
+    uint32_t       reach = have ? 1u << lane : 0u, edges = 0;
+    // the row's members of the piece (undecided neighbours all are): four
+    // neighbours' ids, state words and places in flight at once
+    uint32_t const most = __reduce_max_sync(0xFFFFFFFFu, len);
+    for (uint32_t x = 0; x < most && !left; x += 4) {
+      uint32_t w[4], u[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = x + j < len ? fc[e0 + x + j] : UNDECIDED;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[j] = w[j] != UNDECIDED ? (__ldcg(und + (w[j] >> 5)) >> (w[j] & 31)) & 1u : 0u;
+      // another piece's vertex may just have been decided; one of this piece
+      // has not: the piece is this warp's
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (u[j]) reach |= 1u << (place[w[j]] & 31u), ++edges;
+    }
+    left = left || __reduce_add_sync(0xFFFFFFFFu, edges) > RS_MAXE;
+    if (left) {
+      if (lane == 0) atomicAdd(big, 1u);
+      continue;
+    }
+    // Warshall: after step j every path through places <= j counts
+    for (uint32_t j = 0; j < k; ++j) {
+      uint32_t const rj = __shfl_sync(0xFFFFFFFFu, reach, j);
+      if ((reach >> j) & 1u) reach |= rj;
+    }
+    uint32_t back = 0; // who reaches this lane's vertex
+    for (uint32_t j = 0; j < k; ++j) {
+      unsigned const col = __ballot_sync(0xFFFFFFFFu, (reach >> j) & 1u);
+      if (lane == j) back = col;
+    }
+    uint32_t const scc = reach & back;
+    uint32_t       id  = v;
+    for (uint32_t j = 0; j < k; ++j) {
+      uint32_t const vj = __shfl_sync(0xFFFFFFFFu, v, j);
+      if ((scc >> j) & 1u) id = min(id, vj);
+    }
+    if (have) {
+      scc_id[v] = id;
+      atomicAnd(und + (v >> 5), ~(1u << (v & 31)));
+    }
+    dec += lane == 0 ? k : 0u;
+  }
+  (void)parent;
+  if (lane == 0 && dec) atomicAdd(decided, dec);
+}
+
+// One warp per piece of 33 to RS_MAXV vertices and at most RS_MAXE internal
+// edges; local index = place in the piece.
 __global__ void __launch_bounds__(RS_WARPS * 32)
-k_res_tarjan(uint32_t const* __restrict__ seg_count,
-             uint32_t const* __restrict__ seg_start,
-             uint32_t const* __restrict__ vals,
-             uint64_t const* __restrict__ fh,
-             uint32_t const* __restrict__ fc,
-             uint32_t* und,
-             uint32_t* __restrict__ scc_id,
-             uint32_t* decided,
-             uint32_t* big)
+k_res_tarjan(rs_counts const* __restrict__ rc, uint32_t const* __restrict__ pieces, uint32_t cap, uint32_t const* __restrict__ count, uint32_t const* __restrict__ start,
+             uint32_t const* __restrict__ place, uint32_t const* __restrict__ members, uint64_t const* __restrict__ fh, uint32_t const* __restrict__ fc, uint32_t* und,
+             uint32_t* __restrict__ scc_id, uint32_t* decided, uint32_t* big)
 {
   extern __shared__ __align__(16) unsigned char rs_smem[];
   unsigned const  lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
   rs_piece&       p    = reinterpret_cast<rs_piece*>(rs_smem)[wid];
-  uint32_t const  S    = *seg_count;
+  uint32_t const  S    = rc->mid;
   uint32_t        dec  = 0;
   for (uint32_t sgi = blockIdx.x * RS_WARPS + wid; sgi < S; sgi += gridDim.x * RS_WARPS) {
-    uint32_t const b = seg_start[sgi], k = seg_start[sgi + 1] - b;
-    if (k > RS_MAXV) {
-      if (lane == 0) atomicAdd(big, 1u);
-      continue;
-    }
-    bool heavy_row = false;
+    uint32_t const root = pieces[cap - 1 - sgi], k = count[root], b = start[root];
+    bool           heavy_row = false;
     for (uint32_t i = lane; i < k; i += 32) {
-      uint32_t const v = vals[b + i];
+      uint32_t const v = members[b + i];
       p.vid[i]         = v;
       heavy_row |= fh[v + 1] - fh[v] > HEAVY_ROW;
     }
@@ -284,16 +373,23 @@ k_res_tarjan(uint32_t const* __restrict__ seg_count,
       uint32_t       o = p.off[i];
       for (uint64_t e = fh[v], end = fh[v + 1]; e < end; ++e) {
         uint32_t const w = fc[e];
-        if (und_has(und, w)) p.adj[o++] = static_cast<uint16_t>(rs_local(p, k, w));
+        if (und_has(und, w)) p.adj[o++] = static_cast<uint16_t>(place[w]);
       }
     }
     __syncwarp();
     if (lane == 0) rs_tarjan(p, k);
     __syncwarp();
+    // an SCC's smallest vertex, gathered at its representative in the piece's
+    // spent index / low arrays (16 bits each: a 32-bit slot per vertex)
+    auto* const least = reinterpret_cast<uint32_t*>(p.index);
+    for (uint32_t i = lane; i < k; i += 32) least[i] = UNDECIDED;
+    __syncwarp();
+    for (uint32_t i = lane; i < k; i += 32) atomicMin(least + p.comp[i], p.vid[i]);
+    __syncwarp();
     // ids and und; each vertex's word cleared by an atomic (pieces share words)
     for (uint32_t i = lane; i < k; i += 32) {
       uint32_t const v = p.vid[i];
-      scc_id[v]        = p.vid[p.comp[i]];
+      scc_id[v]        = least[p.comp[i]];
       atomicAnd(und + (v >> 5), ~(1u << (v & 31)));
     }
     dec += lane == 0 ? k : 0;
@@ -306,65 +402,59 @@ k_res_tarjan(uint32_t const* __restrict__ seg_count,
 
 // Decides every undecided piece (weakly connected component of the
 // undecided sub-graph) that fits a warp's shared memory; returns the
-// vertices decided.  *pieces_left (nullable) = pieces left undecided.
+// vertices decided.  `undecided` (n when not known) sizes the launches.  *pieces_left (nullable) = pieces left undecided.
 uint32_t
-residual(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t* pieces_left)
+residual(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t* pieces_left, uint64_t undecided)
 {
   cudaStream_t const s = ctx->stream;
   auto&              ws = ctx->ws;
   if (pieces_left) *pieces_left = 0;
   if (g.n == 0) return 0;
-  uint32_t const words  = (g.n + 31) / 32;
-  size_t const   hist_n = radix_hist_entries(g.n);
-  size_t const   part_n = scan_partial_entries((hist_n > g.n + 1 ? hist_n : g.n + 1) + words + 1);
-  size_t const   hcap   = heavy_capacity(g.n, g.m);
-  size_t const   bytes  = (6 * (static_cast<size_t>(g.n) + 64) + words + 64 + hist_n + part_n + hcap) * sizeof(uint32_t) + 32 * 256;
-  char*          base   = static_cast<char*>(context_buffer(ctx, BUF_BUILD, bytes));
-  size_t         off    = 0;
-  auto           take   = [&](size_t count) {
+  size_t const hcap  = heavy_capacity(g.n, g.m);
+  size_t const each  = static_cast<size_t>(g.n) + 64;
+  size_t const bytes = (6 * each + hcap) * sizeof(uint32_t) + 16 * 256;
+  char*        base  = static_cast<char*>(context_buffer(ctx, BUF_BUILD, bytes));
+  size_t       off   = 0;
+  auto         take  = [&](size_t count) {
     off          = (off + 255) & ~size_t(255);
     auto* const p = reinterpret_cast<uint32_t*>(base + off);
     off += count * sizeof(uint32_t);
     return p;
   };
-  uint32_t* keys = take(g.n + 1);
-  uint32_t* vals = take(g.n + 1);
-  uint32_t* kalt = take(g.n + 1);
-  uint32_t* valt = take(g.n + 1);
-  uint32_t* spos = take(g.n + 2);
-  uint32_t* seg  = take(g.n + 2);
-  uint32_t* wpos = take(words + 1);
-  uint32_t* hist = take(hist_n);
-  uint32_t* part = take(part_n);
-  uint32_t* hlist = take(hcap);
-  uint32_t* parent = ws.label;
+  uint32_t* list    = take(each);
+  uint32_t* count   = take(each); // by vertex: members of the piece whose root it is
+  uint32_t* start   = take(each); // by vertex: a root's range of `members`
+  uint32_t* place   = take(each); // by vertex: its place in its piece
+  uint32_t* members = take(each);
+  uint32_t* pieces  = take(each);
+  uint32_t* hlist   = take(hcap);
+  auto* const rc    = reinterpret_cast<rs_counts*>(take(64));
+  uint32_t* parent  = ws.label;
 
   zero_counters(ctx);
-  unsigned const grid = rs_grid(g.n);
-  k_res_init<<<grid, RS_THREADS, 0, s>>>(g.n, und, parent);
-  k_res_hook<<<grid, RS_THREADS, 0, s>>>(g.n, und, g.fh, g.fc, parent, ws.ctr + CTR_ERR, hlist, ws.ctr + CTR_RES_HEAVY);
-  k_res_hook_heavy<<<148 * 8, RS_THREADS, 0, s>>>(und, g.fh, g.fc, parent, ws.ctr + CTR_ERR, hlist, ws.ctr + CTR_RES_HEAVY);
-  k_res_compress<<<grid, RS_THREADS, 0, s>>>(g.n, und, parent, ws.ctr + CTR_ERR);
-  k_res_flatten<<<grid, RS_THREADS, 0, s>>>(g.n, und, parent, ws.ctr + CTR_ERR);
+  KSPN_CUDA(cudaMemsetAsync(rc, 0, sizeof(rs_counts), s));
+  uint32_t const words = (g.n + 31) / 32;
+  unsigned const grid  = rs_grid(undecided); // passes over the list
+  k_res_list<<<rs_grid(words), RS_THREADS, 0, s>>>(g.n, und, parent, count, list, &rc->list_n);
+  k_res_hook<<<grid, RS_THREADS, 0, s>>>(list, &rc->list_n, und, g.fh, g.fc, parent, ws.ctr + CTR_ERR, hlist, ws.ctr + CTR_RES_HEAVY);
+  if (g.m > HEAVY_ROW) {
+    k_res_hook_heavy<<<std::min<unsigned>(148 * 8, grid * 8), RS_THREADS, 0, s>>>(und, g.fh, g.fc, parent, ws.ctr + CTR_ERR, hlist, ws.ctr + CTR_RES_HEAVY);
+    ctx->launches += 1;
+  }
+  k_res_flatten<<<grid, RS_THREADS, 0, s>>>(list, &rc->list_n, parent, count, place, ws.ctr + CTR_ERR);
+  k_res_ranges<<<grid, RS_THREADS, 0, s>>>(list, parent, count, start, pieces, static_cast<uint32_t>(each), rc, ws.ctr + CTR_AUX);
+  k_res_members<<<grid, RS_THREADS, 0, s>>>(list, &rc->list_n, parent, start, place, members);
+  k_res_small<<<std::min<unsigned>(148 * 8, rs_grid(undecided * 16)), RS_THREADS, 0, s>>>(rc, pieces, count, start, place, parent, members, g.fh, g.fc, und, scc_id, ws.ctr + CTR_DECIDED,
+                                                                                       ws.ctr + CTR_AUX);
+  if (undecided > 32) {
+    size_t const smem = sizeof(rs_piece) * RS_WARPS;
+    KSPN_CUDA(cudaFuncSetAttribute(k_res_tarjan, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    k_res_tarjan<<<static_cast<unsigned>(std::min<uint64_t>(148 * 4, undecided / (33 * RS_WARPS) + 1)), RS_WARPS * 32, smem, s>>>(rc, pieces, static_cast<uint32_t>(each), count, start, place, members, g.fh,
+                                                                                                                      g.fc, und, scc_id, ws.ctr + CTR_DECIDED, ws.ctr + CTR_AUX);
+    ctx->launches += 1;
+  }
   KSPN_CHECK_LAUNCH();
-  // the undecided vertices in id order, then stably by root
-  exclusive_scan<uint32_t>(s, f_und_popc{ und, g.n }, words, wpos, part, &ctx->launches);
-  k_res_list<<<rs_grid(words), RS_THREADS, 0, s>>>(g.n, und, wpos, parent, keys, vals);
-  KSPN_CHECK_LAUNCH();
-  uint32_t k = 0;
-  KSPN_CUDA(cudaMemcpyAsync(&k, wpos + words, sizeof(k), cudaMemcpyDeviceToHost, s));
-  KSPN_CUDA(cudaStreamSynchronize(s));
   ctx->launches += 6;
-  if (k == 0) return 0;
-  radix_sort_pairs(ctx, keys, vals, kalt, valt, k, 0, bits_for(g.n), hist);
-  exclusive_scan<uint32_t>(s, f_seg_head{ keys }, k, spos, part, &ctx->launches);
-  k_res_segments<<<rs_grid(k), RS_THREADS, 0, s>>>(k, keys, spos, seg);
-  // pieces: spos[k] of them, starts in seg
-  size_t const smem = sizeof(rs_piece) * RS_WARPS;
-  KSPN_CUDA(cudaFuncSetAttribute(k_res_tarjan, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  k_res_tarjan<<<148 * 4, RS_WARPS * 32, smem, s>>>(spos + k, seg, vals, g.fh, g.fc, und, scc_id, ws.ctr + CTR_DECIDED, ws.ctr + CTR_AUX);
-  KSPN_CHECK_LAUNCH();
-  ctx->launches += 2;
   read_counters(ctx);
   if (ctx->h_ctr[CTR_ERR]) throw error{ KSPN_ERR_INTERNAL, "residual: union-find loop bound reached" };
   if (pieces_left) *pieces_left = ctx->h_ctr[CTR_AUX];

@@ -1087,18 +1087,17 @@ select_pivot_live(kspn_context* ctx, dgraph const& g, uint32_t const* und)
   return (prod == 0 || p == NONE) ? g.n : p;
 }
 
-uint32_t
-count_undecided(kspn_context* ctx, uint32_t n, uint32_t const* und)
+void
+count_undecided_async(kspn_context* ctx, uint32_t n, uint32_t const* und)
 {
-  uint32_t const words = (n + 31) / 32;
-  zero_counters(ctx);
+  uint32_t const  words = (n + 31) / 32;
+  uint32_t* const left  = ctx->ws.ctr + CTR_LEFT;
+  KSPN_CUDA(cudaMemsetAsync(left, 0, sizeof(uint32_t), ctx->stream));
   if (words) {
-    k_popcount<<<stream_grid(words), T_THREADS, 0, ctx->stream>>>(words, n, und, ctx->ws.ctr + CTR_AUX);
+    k_popcount<<<stream_grid(words), T_THREADS, 0, ctx->stream>>>(words, n, und, left);
     KSPN_CHECK_LAUNCH();
     ctx->launches += 1;
   }
-  read_counters(ctx);
-  return ctx->h_ctr[CTR_AUX];
 }
 
 } // namespace kspn
