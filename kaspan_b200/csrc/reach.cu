@@ -694,7 +694,10 @@ k_bu_cut_clear(gate g, bu_cut cut)
 // Vertices per start vertex of a worklist phase (run_async).  RGG of 10^6 /
 // 60,000 vertices, whole call: 2048: 1.56 / 1.07 ms, 4096: 1.51 / 0.91,
 // 8192: 1.90 / 1.34; 2^24 vertices (255 start vertices each way): the same.
-constexpr uint32_t SEED_SPAN       = 4096;
+// Below SEED_MIN of them the pivot alone starts: a restart (one start vertex
+// in four not shown to belong) costs what the others save (RGG of 20,000
+// vertices: 0.85 ms with 4 and no restart, 1.37 with one, 1.1 without any).
+constexpr uint32_t SEED_SPAN       = 4096, SEED_MIN = 8;
 constexpr unsigned GRID_SYNC_SPINS = 1u << 22; // default wait limit (kspn_options.wait_limit = 0)
 
 // Grid barrier with a monotonically growing counter: every block adds 1
@@ -2843,7 +2846,7 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
   a.resume       = 0;
   // start vertices for a worklist phase: one per SEED_SPAN vertices (a hop
   // costs the same for one or hundreds of searches in flight)
-  a.seeds        = g.m < (1ull << 31) ? std::min<uint32_t>(255, g.n / SEED_SPAN) : 0u;
+  a.seeds        = g.m < (1ull << 31) && g.n / SEED_SPAN >= SEED_MIN ? std::min<uint32_t>(255, g.n / SEED_SPAN) : 0u;
   a.seed_n       = pivot_candidates(g.n);
   a.seed_ids     = reinterpret_cast<uint32_t const*>(ws.pivot + 4096);
   a.label        = reinterpret_cast<uint8_t*>(ws.label);

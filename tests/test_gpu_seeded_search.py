@@ -1,5 +1,5 @@
 """Worklist phases that start from several vertices: long, thin graphs of
-enough vertices for 2 to 40 start vertices, all of them in the pivot's SCC,
+enough vertices for 8 to 73 start vertices, all of them in the pivot's SCC,
 some of them, or none; and every take policy of the worklist.  Output
 bit-identical to the oracle's Tarjan."""
 from __future__ import annotations
@@ -19,8 +19,9 @@ N, SETS, SIZE = 100000, 12, 400
 
 def build(kind):
     """A long cycle holding the pivot, and SETS small components whose
-    vertices have the largest in * out of their 1024 ids: with N vertices, 12
-    start vertices are tried, each the best of one such stretch."""
+    vertices have the largest in * out of their 1024 ids: with N vertices, 24
+    start vertices are tried, each the best of one such stretch, every other
+    one of them in a set."""
     rng = np.random.default_rng(3)
     if kind == "grid":  # a sparse directed grid, many small components around a large one
         w = 300
@@ -78,7 +79,7 @@ def test_matches_tarjan(ctx, kind, after):
             assert st.as_dict()["search_worklist"] == 1
 
 
-@pytest.mark.parametrize("n", [16383, 16384, 24576, 65535, 300007])
+@pytest.mark.parametrize("n", [16384, 32767, 32768, 65535, 300007])
 def test_rgg_sizes(ctx, n):
     import torch
 
