@@ -282,7 +282,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
     while (decided < g.n) {
       if (st && st->label_calls >= round_cap) throw error{ KSPN_ERR_TIMEOUT, "label-search call cap exceeded" };
       label_ran = true;
-      add(KSPN_PHASE_LABEL, label_search(ctx, g, und, scc_id, ++rotation, opt, st));
+      add(KSPN_PHASE_LABEL, label_search(ctx, g, und, scc_id, ++rotation, opt, st, g.n - decided));
     }
   } else if (opt.pipeline != KSPN_PIPELINE_FAST) {
     // the reference's variants (variant/*.hpp), phase order at one rank
@@ -293,7 +293,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
       while (decided < g.n) {
         if (++calls > round_cap) throw error{ KSPN_ERR_TIMEOUT, "label-search call cap exceeded" };
         label_ran = true;
-        add(KSPN_PHASE_LABEL, label_search(ctx, g, und, scc_id, ++rotation, opt, st));
+        add(KSPN_PHASE_LABEL, label_search(ctx, g, und, scc_id, ++rotation, opt, st, g.n - decided));
         if (trim_between && decided < g.n) add(KSPN_PHASE_TRIM, trim_fixpoint(ctx, g, und, scc_id, false, 0));
       }
     };
@@ -462,7 +462,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
       }
       if (decided < g.n) {
         label_ran = true;
-        add(KSPN_PHASE_LABEL, label_search(ctx, g, und, scc_id, ++rotation, opt, st));
+        add(KSPN_PHASE_LABEL, label_search(ctx, g, und, scc_id, ++rotation, opt, st, g.n - decided));
       }
     }
     if (st) st->rounds = rounds;
@@ -948,7 +948,7 @@ kspn_label_search(kspn_context* ctx, uint32_t n, uint64_t m, const uint64_t* d_f
     kspn_options o;
     kspn_options_default(&o);
     dgraph const   g{ n, m, d_fw_head, d_fw_csr, d_bw_head, d_bw_csr };
-    uint32_t const d = n ? label_search(ctx, g, reinterpret_cast<uint32_t*>(d_undecided), d_scc_id, rotation, o, nullptr) : 0;
+    uint32_t const d = n ? label_search(ctx, g, reinterpret_cast<uint32_t*>(d_undecided), d_scc_id, rotation, o, nullptr, ~0ull) : 0; // (d_label holds every vertex: the general path)
     if (d_label && n) KSPN_CUDA(cudaMemcpyAsync(d_label, ctx->ws.label, static_cast<size_t>(n) * 4, cudaMemcpyDeviceToDevice, ctx->stream));
     KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
     if (decided) *decided = d;

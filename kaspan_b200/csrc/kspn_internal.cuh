@@ -538,7 +538,8 @@ void   release_graphs(kspn_context* ctx);
 uint32_t fw_bw(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t pivot, kspn_options const& opt, kspn_stats* st, bool min_ids);
 
 // label.cu
-uint32_t label_search(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, int rotation, kspn_options const& opt, kspn_stats* st);
+// undecided: how many vertices are (any larger number if not known)
+uint32_t label_search(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, int rotation, kspn_options const& opt, kspn_stats* st, uint64_t undecided);
 
 // canon.cu
 // members: every id is a member of its own class (pipeline output); else

@@ -183,10 +183,195 @@ struct label_bw_op
   }
 };
 
+// ---------------------------------------------------------------- few undecided vertices
+// A search over at most LS_VERTICES undecided vertices with at most LS_EDGES
+// row entries runs in one block after one listing pass: level after level
+// behind block barriers, instead of four launches, a memset and a host round
+// trip per level (about 35 us each; a near-critical random graph of 10^6
+// vertices left 10,248 vertices and ~490 levels: 17.2 ms).  A level costs
+// its chain of dependent accesses, 3 to 4 us.
+constexpr int      LS_THREADS  = 1024;
+constexpr uint32_t LS_VERTICES = 1u << 15;
+constexpr uint64_t LS_EDGES    = 1u << 20;
+constexpr uint32_t LS_ROW      = 8192; // longest row one warp walks
+
+struct ls_counts
+{
+  uint32_t           list_n, longest;
+  unsigned long long entries; // out- and in-row entries of the listed vertices
+  uint32_t           ran;     // 0: over the limits, nothing done
+  uint32_t           err;     // 1: propagation cap, 2: closure cap
+  uint32_t           decided;
+  uint32_t           pad;
+  unsigned long long edges;   // row entries walked
+};
+
+// The undecided vertices with their first labels, and the size of their rows.
+__global__ void __launch_bounds__(L_THREADS)
+k_label_list(uint32_t n, uint32_t const* __restrict__ und, uint64_t const* __restrict__ fh, uint64_t const* __restrict__ bh, uint32_t* __restrict__ label, uint32_t* __restrict__ stamp, seed_map sm,
+             uint32_t* __restrict__ list, ls_counts* lc)
+{
+  unsigned const lane  = threadIdx.x & 31u;
+  uint32_t const words = (n + 31) / 32, span = (words + 31) & ~31u;
+  for (uint32_t w = blockIdx.x * L_THREADS + threadIdx.x; w < span; w += gridDim.x * L_THREADS) {
+    uint32_t x = w < words ? und[w] : 0u;
+    if (w == words - 1 && (n & 31)) x &= (1u << (n & 31)) - 1u;
+    uint32_t const c    = __popc(x);
+    uint32_t       incl = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      uint32_t const y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= static_cast<unsigned>(d)) incl += y;
+    }
+    uint32_t const tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    if (!tot) continue; // warp-uniform
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&lc->list_n, tot);
+    at = __shfl_sync(0xFFFFFFFFu, at, 0) + incl - c;
+    unsigned long long entries = 0;
+    uint32_t           longest = 0;
+    for (; x; x &= x - 1) {
+      uint32_t const v = w * 32 + __ffs(x) - 1;
+      uint64_t const o = fh[v + 1] - fh[v], i = bh[v + 1] - bh[v];
+      list[at++]       = v;
+      label[v]         = sm.map(v);
+      stamp[v]         = 0;
+      entries += o + i;
+      longest = max(longest, static_cast<uint32_t>(min(max(o, i), static_cast<uint64_t>(UNDECIDED))));
+    }
+    if (entries) atomicAdd(&lc->entries, entries), atomicMax(&lc->longest, longest);
+  }
+}
+
+// hit(u, w) for every neighbour w of list[0, cnt)'s rows; the accepted ones
+// are appended to out.  A warp takes 32 listed vertices; its lanes share the
+// entries of their rows.
+template<class F>
+__device__ __forceinline__ void
+ls_expand(uint32_t const* list, uint32_t cnt, uint64_t const* __restrict__ head, uint32_t const* __restrict__ adj, uint32_t* out, uint32_t* counter, unsigned long long& edges, F&& hit)
+{
+  unsigned const lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  for (uint32_t i0 = threadIdx.x & ~31u; i0 < cnt; i0 += LS_THREADS) {
+    bool const     ok   = i0 + lane < cnt;
+    uint32_t const u    = ok ? __ldcg(list + i0 + lane) : 0u;
+    uint64_t const b    = ok ? head[u] : 0ull;
+    uint32_t const len  = ok ? static_cast<uint32_t>(head[u + 1] - b) : 0u;
+    uint32_t       incl = len;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      uint32_t const y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= static_cast<unsigned>(d)) incl += y;
+    }
+    uint32_t const tot = __shfl_sync(0xFFFFFFFFu, incl, 31), excl = incl - len;
+    edges += len;
+    for (uint32_t e0 = 0; e0 < tot; e0 += 32) {
+      uint32_t const e = e0 + lane;
+      uint32_t       j = 0;
+#pragma unroll
+      for (int step = 16; step; step >>= 1)
+        if (__shfl_sync(0xFFFFFFFFu, excl, j + step) <= e) j += step;
+      uint64_t const bj = __shfl_sync(0xFFFFFFFFu, b, j);
+      uint32_t const xj = __shfl_sync(0xFFFFFFFFu, excl, j), uj = __shfl_sync(0xFFFFFFFFu, u, j);
+      uint32_t const w  = e < tot ? adj[bj + (e - xj)] : 0u;
+      bool const     f  = e < tot && hit(uj, w);
+      unsigned const m  = __ballot_sync(0xFFFFFFFFu, f);
+      if (!m) continue;
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(counter, static_cast<uint32_t>(__popc(m)));
+      at = __shfl_sync(0xFFFFFFFFu, at, 0);
+      if (f) __stcg(out + at + __popc(m & lt), w);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(LS_THREADS)
+k_label_small(uint64_t const* __restrict__ fh, uint32_t const* __restrict__ fc, uint64_t const* __restrict__ bh, uint32_t const* __restrict__ bc, uint32_t* und, uint32_t* label, uint32_t* stamp,
+              uint32_t* __restrict__ scc_id, seed_map sm, uint32_t const* list, uint32_t* q0, uint32_t* q1, uint32_t cap, ls_counts* lc)
+{
+  __shared__ uint32_t           s_n[3]; // append counters by level: used, next, being cleared
+  __shared__ unsigned long long s_edges;
+  uint32_t const k = lc->list_n;
+  if (k > LS_VERTICES || lc->entries > LS_EDGES || lc->longest > LS_ROW) return;
+  if (threadIdx.x < 3) s_n[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_edges = 0;
+  __syncthreads();
+  unsigned long long edges = 0;
+  uint32_t           level = 0, err = 0;
+  uint32_t*          q[2]  = { q0, q1 };
+  // ends a level: its appended count (one barrier; see the counters)
+  auto const close = [&]() {
+    __syncthreads();
+    uint32_t const c = s_n[level % 3];
+    if (threadIdx.x == 0) s_n[(level + 2) % 3] = 0;
+    ++level;
+    return c;
+  };
+  // forward: the min-label fixpoint
+  uint32_t const* cur = list;
+  for (uint32_t cnt = k; cnt;) {
+    if (level >= cap) {
+      err = 1;
+      break;
+    }
+    uint32_t* const nxt = q[level & 1];
+    ls_expand(cur, cnt, fh, fc, nxt, &s_n[level % 3], edges, [&](uint32_t u, uint32_t v) {
+      if (!((__ldcg(und + (v >> 5)) >> (v & 31)) & 1u)) return false;
+      uint32_t const lu = __ldcg(label + u);
+      if (lu >= __ldcg(label + v) || lu >= atomicMin(label + v, lu)) return false;
+      return atomicExch(stamp + v, level + 1) != level + 1; // once per level
+    });
+    cnt = close();
+    cur = nxt;
+  }
+  // roots, then the backward closure inside each label class
+  uint32_t decided = 0, base = level;
+  if (!err) {
+    uint32_t* const nxt = q[level & 1];
+    for (uint32_t i0 = threadIdx.x & ~31u; i0 < k; i0 += LS_THREADS) {
+      unsigned const lane = threadIdx.x & 31u;
+      uint32_t const v    = i0 + lane < k ? __ldcg(list + i0 + lane) : UNDECIDED;
+      bool const     root = v != UNDECIDED && __ldcg(label + v) == sm.map(v);
+      if (root) {
+        bit_take(und, v);
+        scc_id[v] = v;
+      }
+      unsigned const m  = __ballot_sync(0xFFFFFFFFu, root);
+      uint32_t       at = 0;
+      if (lane == 0 && m) at = atomicAdd(&s_n[level % 3], static_cast<uint32_t>(__popc(m)));
+      at = __shfl_sync(0xFFFFFFFFu, at, 0);
+      if (root) __stcg(nxt + at + __popc(m & ((1u << lane) - 1u)), v);
+    }
+    uint32_t cnt = close();
+    decided      = cnt;
+    cur          = nxt;
+    base         = level;
+    while (cnt) {
+      if (level - base >= cap) {
+        err = 2;
+        break;
+      }
+      uint32_t* const to = q[level & 1];
+      ls_expand(cur, cnt, bh, bc, to, &s_n[level % 3], edges, [&](uint32_t u, uint32_t v) {
+        if (!((__ldcg(und + (v >> 5)) >> (v & 31)) & 1u)) return false;
+        uint32_t const lu = __ldcg(label + u);
+        if (__ldcg(label + v) != lu || !bit_take(und, v)) return false;
+        scc_id[v] = sm.unmap(lu);
+        return true;
+      });
+      cnt = close();
+      decided += cnt;
+      cur = to;
+    }
+  }
+  if (edges) atomicAdd(&s_edges, edges);
+  __syncthreads();
+  if (threadIdx.x == 0) lc->ran = 1, lc->err = err, lc->decided = decided, lc->edges = s_edges;
+}
+
 } // namespace
 
 uint32_t
-label_search(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, int rotation, kspn_options const& opt, kspn_stats* st)
+label_search(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, int rotation, kspn_options const& opt, kspn_stats* st, uint64_t undecided)
 {
   auto&          ws    = ctx->ws;
   size_t const   words = (static_cast<size_t>(g.n) + 31) / 32;
@@ -205,6 +390,25 @@ label_search(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id
     KSPN_CHECK_LAUNCH();
     ctx->launches += 1;
     sm = seed_map{ bk, rotation, shift, (static_cast<uint32_t>(rotation) * 0x9E3779B9u) & ((1u << shift) - 1u) };
+  }
+  if (undecided <= LS_VERTICES && !ctx->prof) {
+    // few vertices: one block, unless their rows are too many or too long
+    auto* const lc = reinterpret_cast<ls_counts*>(ws.links);
+    ls_counts   h{};
+    KSPN_CUDA(cudaMemsetAsync(lc, 0, sizeof(ls_counts), ctx->stream));
+    k_label_list<<<l_grid((g.n + 31) / 32), L_THREADS, 0, ctx->stream>>>(g.n, und, g.fh, g.bh, ws.label, ws.indeg, sm, ws.q2, lc);
+    k_label_small<<<1, LS_THREADS, 0, ctx->stream>>>(g.fh, g.fc, g.bh, g.bc, und, ws.label, ws.indeg, scc_id, sm, ws.q2, ws.q0, ws.q1, cap, lc);
+    KSPN_CHECK_LAUNCH();
+    ctx->launches += 2;
+    KSPN_CUDA(cudaMemcpyAsync(&h, lc, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+    KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (h.ran) {
+      if (h.err == 1) throw error{ KSPN_ERR_TIMEOUT, "label search: propagation cap exceeded" };
+      if (h.err == 2) throw error{ KSPN_ERR_TIMEOUT, "label search: closure cap exceeded" };
+      ctx->td_edges += h.edges;
+      if (st) st->label_calls += 1;
+      return h.decided;
+    }
   }
   zero_counters(ctx);
   KSPN_CUDA(cudaMemsetAsync(ws.vis_a, 0, words * 4, ctx->stream));
