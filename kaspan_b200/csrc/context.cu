@@ -254,7 +254,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
   // with its results: no host round trip of their own
   bool const resident = opt.pipeline == KSPN_PIPELINE_FAST && g.n != 0 && !ctx->prof && resident_fits(g);
   if (opt.validate) {
-    if (resident) validate_async(ctx, g, !own_transpose);
+    if (resident) validate_async(ctx, g, !own_transpose, false); // trim_1_first reads the offsets
     else validate(ctx, g, !own_transpose);
   }
   if (g.n == 0) return;
@@ -373,7 +373,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
     if (resident) {
       // trim_1_first, then FW-BW and the trim fixpoint in ONE persistent
       // launch that takes the pivot from device memory: one host sync
-      trim_1_first_async(ctx, g, und);
+      trim_1_first_async(ctx, g, und, opt.validate != 0);
       KSPN_CUDA(cudaEventRecord(ctx->ev[2], ctx->stream));
       // with the learned rule the launch first scores the plain pivot (no
       // extra launch when the model accepts it)

@@ -183,13 +183,16 @@ k_edges_to_csr(uint32_t n, uint64_t m_raw, uint64_t chunk, uint32_t const* __res
 }
 
 // One direction's checks per grid row (blockIdx.y: CSR, transpose), both in
-// one launch.  A pure stream: 8(n+1) + 4m bytes per direction, so the ids
-// are read 16 bytes at a time with VA_ILP loads in flight per thread (the
-// rows' array may start at any 4-byte address: the ids before the first and
-// after the last 16-byte boundary are read one by one).  R-MAT scale 24
-// (n 16.8 M, m 263 M), per direction: 443 us with one 4-byte load per
-// thread and step, 245 us this way.
-constexpr int VA_THREADS = 256, VA_ILP = 4;
+// one launch.  A pure stream of 4m bytes per direction, and 8(n+1) more with
+// `heads` (false: k_trim_first, which reads every offset next, checks them).
+// The ids are read 16 bytes at a time with VA_ILP loads in flight per thread
+// (the rows' array may start at any 4-byte address: the ids before the first
+// and after the last 16-byte boundary are read one by one).  R-MAT scale 24
+// (n 16.8 M, m 263 M), both directions: 886 us with one 4-byte load per
+// thread and step, 490 us with 4 x 16 bytes and the offsets; ids alone 470 us
+// with 4 x 16 bytes, 345 us with 8 (6.1 TB/s; 16: 340 us), which need the
+// grid of 4 blocks per SM and row or more (2: 470 us, 3: 365 us).
+constexpr int VA_THREADS = 256, VA_ILP = 8;
 struct graph_rows
 {
   uint64_t const* head;
@@ -197,13 +200,13 @@ struct graph_rows
 };
 
 __global__ void __launch_bounds__(VA_THREADS)
-k_validate(uint32_t n, uint64_t m, graph_rows fw, graph_rows bw, uint32_t* __restrict__ err)
+k_validate(uint32_t n, uint64_t m, graph_rows fw, graph_rows bw, bool heads, uint32_t* __restrict__ err)
 {
   graph_rows const g      = blockIdx.y ? bw : fw;
   uint64_t const   stride = static_cast<uint64_t>(gridDim.x) * VA_THREADS;
   uint64_t const   tid    = static_cast<uint64_t>(blockIdx.x) * VA_THREADS + threadIdx.x;
   uint32_t         bad    = 0;
-  for (uint64_t i0 = tid; i0 < n; i0 += VA_ILP * stride) {
+  for (uint64_t i0 = heads ? tid : n; i0 < n; i0 += VA_ILP * stride) {
     uint64_t a[VA_ILP], b[VA_ILP];
 #pragma unroll
     for (int k = 0; k < VA_ILP; ++k) {
@@ -214,7 +217,7 @@ k_validate(uint32_t n, uint64_t m, graph_rows fw, graph_rows bw, uint32_t* __res
 #pragma unroll
     for (int k = 0; k < VA_ILP; ++k) bad |= a[k] > b[k] ? 1u : 0u;
   }
-  if (tid == 0 && (g.head[0] != 0 || g.head[n] != m)) bad |= 2u;
+  if (heads && tid == 0 && (g.head[0] != 0 || g.head[n] != m)) bad |= 2u;
   uint64_t const lead = min(m, ((16u - (reinterpret_cast<uintptr_t>(g.csr) & 15u)) & 15u) / 4u);
   uint64_t const nv   = (m - lead) / 4;
   auto const*    v    = reinterpret_cast<uint4 const*>(g.csr + lead);
@@ -611,11 +614,11 @@ build_csr(kspn_context* ctx, uint32_t n, uint64_t m_raw, uint32_t* src, uint32_t
 }
 
 void
-validate_async(kspn_context* ctx, dgraph const& g, bool transpose_too)
+validate_async(kspn_context* ctx, dgraph const& g, bool transpose_too, bool heads)
 {
   uint64_t const items = std::max<uint64_t>(g.m / (4 * VA_ILP), g.n / VA_ILP) + 1;
-  unsigned const gx    = static_cast<unsigned>(std::min<uint64_t>(div_up(items, VA_THREADS), 148ull * 4)); // both directions resident at once
-  k_validate<<<dim3(gx, transpose_too && g.bh != g.fh ? 2 : 1), VA_THREADS, 0, ctx->stream>>>(g.n, g.m, graph_rows{ g.fh, g.fc }, graph_rows{ g.bh, g.bc }, ctx->ws.ctr + CTR_ERR);
+  unsigned const gx    = static_cast<unsigned>(std::min<uint64_t>(div_up(items, VA_THREADS), 148ull * 8)); // both directions resident at once
+  k_validate<<<dim3(gx, transpose_too && g.bh != g.fh ? 2 : 1), VA_THREADS, 0, ctx->stream>>>(g.n, g.m, graph_rows{ g.fh, g.fc }, graph_rows{ g.bh, g.bc }, heads, ctx->ws.ctr + CTR_ERR);
   KSPN_CHECK_LAUNCH();
   ctx->launches += 1;
 }
@@ -635,7 +638,7 @@ void
 validate(kspn_context* ctx, dgraph const& g, bool transpose_too)
 {
   KSPN_CUDA(cudaMemsetAsync(ctx->ws.ctr + CTR_ERR, 0, sizeof(uint32_t), ctx->stream));
-  validate_async(ctx, g, transpose_too);
+  validate_async(ctx, g, transpose_too, true);
   read_counters(ctx);
   validate_check(ctx->h_ctr[CTR_ERR]);
 }

@@ -498,7 +498,7 @@ resident_result fw_bw_trim_result(kspn_context* ctx, dgraph const& g, kspn_optio
 std::pair<uint32_t, uint32_t> fw_bw_trim(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t pivot, kspn_options const& opt, kspn_stats* st);
 
 uint32_t trim_1_first(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t* queue_out, uint32_t* queue_count_host, bool init_degrees);
-void     trim_1_first_async(kspn_context* ctx, dgraph const& g, uint32_t* und); // ws.ctr zeroed by the caller; writes no ids; no host sync: decided in ws.ctr, pivot in PV_FINAL
+void     trim_1_first_async(kspn_context* ctx, dgraph const& g, uint32_t* und, bool check); // check: the offsets' fault bits into ws.ctr[CTR_ERR]; ws.ctr zeroed by the caller; writes no ids; no host sync: decided in ws.ctr, pivot in PV_FINAL
 uint32_t trim_1_normal(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id);
 uint32_t trim_fixpoint(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, bool degrees_from_first, uint32_t seed_count);
 uint32_t trim_exhaustive_first(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t* outdeg, uint32_t* indeg);
@@ -565,7 +565,7 @@ uint64_t build_csr(kspn_context* ctx, uint32_t n, uint64_t m_raw, uint32_t* src,
 // host has read them.  transpose_too: false when the transpose was built
 // here from the checked CSR.
 void     validate(kspn_context* ctx, dgraph const& g, bool transpose_too = true);
-void     validate_async(kspn_context* ctx, dgraph const& g, bool transpose_too);
+void     validate_async(kspn_context* ctx, dgraph const& g, bool transpose_too, bool heads); // heads: the offsets too
 void     validate_check(uint32_t e);
 
 // gen.cu

@@ -184,6 +184,11 @@ k_pv_final(uint32_t nb, uint64_t* prod, uint32_t* id)
 // ---------------------------------------------------------------- trim_1_first
 constexpr int TF_ITEMS = 4; // vertices per thread per pass of k_trim_first
 
+// CHECK: the offset arrays are checked on the way, with k_validate's fault
+// bits.  A template parameter: as a run-time flag the kernel without checks
+// took 258 instead of 210 us on R-MAT scale 26 (1.07 GB of offsets; taking
+// f1, b1 from the next lane by shuffle: 255 us; TF_ITEMS 2: 220, 8: 280).
+template<bool CHECK>
 __global__ void __launch_bounds__(T_THREADS)
 k_trim_first(uint32_t n,
              uint64_t const* __restrict__ fh,
@@ -195,7 +200,9 @@ k_trim_first(uint32_t n,
              uint32_t* __restrict__ queue,
              uint32_t* __restrict__ ctr,
              uint64_t* __restrict__ blk_prod,
-             uint32_t* __restrict__ blk_id)
+             uint32_t* __restrict__ blk_id,
+             uint64_t m,
+             uint32_t* __restrict__ err)
 {
   __shared__ uint32_t s_buf[DENSE_BUF];
   __shared__ uint32_t s_n, s_base;
@@ -204,6 +211,7 @@ k_trim_first(uint32_t n,
   block_queue    bq{ s_buf, &s_n };
   pv             best = { 0, NONE };
   uint32_t       dec  = 0;
+  uint32_t       bad  = 0;
   // a pass covers TF_ITEMS slices of T_THREADS vertices; all offset loads
   // of a pass are issued before any is used
   uint64_t const pass     = static_cast<uint64_t>(T_THREADS) * TF_ITEMS;
@@ -220,6 +228,10 @@ k_trim_first(uint32_t n,
       uint64_t const t       = base + k * T_THREADS + threadIdx.x;
       uint32_t const v       = static_cast<uint32_t>(t);
       bool const     valid   = t < n;
+      if constexpr (CHECK) {
+        if (f0[k] > f1[k] || b0[k] > b1[k]) bad |= 1u;
+        if ((t == 0 && (f0[k] | b0[k])) || (t + 1 == n && (f1[k] != m || b1[k] != m))) bad |= 2u;
+      }
       uint64_t const out     = f1[k] - f0[k];
       uint64_t const in      = b1[k] - b0[k];
       bool const     trimmed = valid && (in == 0 || out == 0);
@@ -242,6 +254,7 @@ k_trim_first(uint32_t n,
     }
   }
   if (queue) bq.flush(queue, ctr + CTR_Q0, &s_base);
+  if (CHECK && bad) atomicOr(err, bad);
   // decided count
   unsigned d = dec;
 #pragma unroll
@@ -917,7 +930,7 @@ trim_1_first(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id
   zero_counters(ctx);
   unsigned const nb = pivot_candidates(g.n);
   prof_start(ctx);
-  k_trim_first<<<nb, T_THREADS, 0, ctx->stream>>>(g.n, g.fh, g.bh, und, scc_id, init_degrees ? ws.indeg : nullptr, init_degrees ? ws.outdeg : nullptr, queue_out, ws.ctr, ws.pivot, reinterpret_cast<uint32_t*>(ws.pivot + 4096));
+  k_trim_first<false><<<nb, T_THREADS, 0, ctx->stream>>>(g.n, g.fh, g.bh, und, scc_id, init_degrees ? ws.indeg : nullptr, init_degrees ? ws.outdeg : nullptr, queue_out, ws.ctr, ws.pivot, reinterpret_cast<uint32_t*>(ws.pivot + 4096), g.m, nullptr);
   prof_stop(ctx);
   KSPN_CHECK_LAUNCH();
   ctx->launches += 1;
@@ -946,7 +959,7 @@ pivot_candidates(uint32_t n)
   static unsigned const wave = [] {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trim_first, T_THREADS, 0) != cudaSuccess || per_sm <= 0) per_sm = 4;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trim_first<true>, T_THREADS, 0) != cudaSuccess || per_sm <= 0) per_sm = 4;
     return static_cast<unsigned>(std::min(sms * per_sm, static_cast<int>(PV_FINAL)));
   }();
   uint64_t const b = (static_cast<uint64_t>(n) + static_cast<uint64_t>(T_THREADS) * TF_ITEMS - 1) / (static_cast<uint64_t>(T_THREADS) * TF_ITEMS);
@@ -956,11 +969,12 @@ pivot_candidates(uint32_t n)
 // (the caller has zeroed ws.ctr; ids are not written: the resident
 // launch that follows writes every vertex's id at its end)
 void
-trim_1_first_async(kspn_context* ctx, dgraph const& g, uint32_t* und)
+trim_1_first_async(kspn_context* ctx, dgraph const& g, uint32_t* und, bool check)
 {
   auto& ws = ctx->ws;
   prof_start(ctx);
-  k_trim_first<<<pivot_candidates(g.n), T_THREADS, 0, ctx->stream>>>(g.n, g.fh, g.bh, und, nullptr, nullptr, nullptr, nullptr, ws.ctr, ws.pivot, reinterpret_cast<uint32_t*>(ws.pivot + 4096));
+  auto kernel = check ? k_trim_first<true> : k_trim_first<false>;
+  kernel<<<pivot_candidates(g.n), T_THREADS, 0, ctx->stream>>>(g.n, g.fh, g.bh, und, nullptr, nullptr, nullptr, nullptr, ws.ctr, ws.pivot, reinterpret_cast<uint32_t*>(ws.pivot + 4096), g.m, ws.ctr + CTR_ERR);
   prof_stop(ctx);
   KSPN_CHECK_LAUNCH();
   ctx->launches += 1;
