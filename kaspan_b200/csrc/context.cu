@@ -221,6 +221,45 @@ struct phase_clock
   }
 };
 
+// The graph in one block, if its size and the options allow: the FAST
+// pipeline with its own pivot, without the caps and hooks of the grid-wide
+// launches.  False: not run (or, unchecked, the arrays are not a plain CSR
+// pair of m entries), nothing written that the grid-wide path does not write.
+bool
+run_small(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options const& opt, kspn_stats* st)
+{
+  if (opt.pipeline != KSPN_PIPELINE_FAST || ctx->union_route || (opt.learned_pivot && ctx->pivot_model) || opt.profile || opt.trace || opt.max_levels || opt.max_rounds || opt.wait_limit ||
+      opt.drop_barrier || opt.aw_exact_after || !small_fits(g))
+    return false;
+  auto* const res = reinterpret_cast<small_result*>(static_cast<char*>(ctx->h_state) + SMALL_RESULT_AT);
+  if (st) KSPN_CUDA(cudaEventRecord(ctx->ev[0], ctx->stream));
+  scc_small_async(ctx, g, scc_id, res);
+  if (st) KSPN_CUDA(cudaEventRecord(ctx->ev[1], ctx->stream));
+  KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
+  look_back_check(ctx);
+  if (res->bad) {
+    if (opt.validate) validate_check(res->bad);
+    return false;
+  }
+  if (static_cast<uint64_t>(res->trim_first) + res->fwbw + res->trim + res->rest != g.n) throw error{ KSPN_ERR_INTERNAL, "decided-vertex count does not match n" };
+  if (st) {
+    float ms = 0;
+    KSPN_CUDA(cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
+    st->ms_total = st->ms[KSPN_PHASE_FWBW]  = ms; // one launch: not split further
+    st->decided[KSPN_PHASE_TRIM_FIRST]      = res->trim_first;
+    st->decided[KSPN_PHASE_FWBW]            = res->fwbw;
+    st->decided[KSPN_PHASE_TRIM]            = res->trim;
+    st->decided[KSPN_PHASE_RESIDUAL]        = res->rest;
+    st->pivot                               = res->pivot;
+    st->levels_fw                           = res->levels_fw;
+    st->levels_bw                           = res->levels_bw;
+    st->edges_scanned                       = res->edges;
+    st->rounds                              = 1;
+    st->kernel_launches                     = 1;
+  }
+  return true;
+}
+
 // The whole path on a resident graph; writes the canonical ids into scc_id.
 // own_transpose: (bh, bc) was built here from the CSR, so checking the CSR
 // checks it too (a transpose of valid rows is valid).
@@ -235,6 +274,7 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
     st->m     = g.m;
     st->pivot = g.n;
   }
+  if (run_small(ctx, g, scc_id, opt, st)) return;
   uint64_t const launches0 = ctx->launches;
   KSPN_CUDA(cudaMemsetAsync(ws.ctr, 0, 64 * sizeof(uint32_t), ctx->stream));
   std::memset(ctx->h_ctr, 0, 64 * sizeof(uint32_t));

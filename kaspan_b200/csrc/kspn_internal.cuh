@@ -400,6 +400,7 @@ struct kspn_context
   cudaStream_t       stream     = nullptr;
   bool               own_stream = false;
   kspn::workspace    ws;
+  bool               small_ready = false; // k_scc_small's shared-memory limit is set on this device
   uint32_t*          h_ctr      = nullptr; // pinned mirror of ws.ctr
   uint64_t*          h_ctr64    = nullptr;
   int                rotation   = 0; // label-search calls made by this context
@@ -410,7 +411,7 @@ struct kspn_context
   // kernel-class timing (kspn_options.profile): two event pairs in flight
   kspn_stats*        prof       = nullptr;
   cudaEvent_t        pe[4]      = {};
-  void*              h_state    = nullptr; // pinned 4 KiB mirror of ws.rstate
+  void*              h_state    = nullptr; // pinned 4 KiB: mirror of ws.rstate, trim state at 512, small_result at SMALL_RESULT_AT, look-back fault word last
   unsigned           search_grid = 0;      // blocks of the persistent FW-BW launch
   unsigned           resume_grid = 0;      // blocks of its resume launch (the worklist phase)
   unsigned           bar_grid    = 0;      // grid of the last launch on the workspace's grid barrier
@@ -491,6 +492,17 @@ struct resident_result
   bool     resumed        = false; // the worklist phase ran in a resume launch (after one more host round trip) // the pivot model rejected trim_1_first's pivot: the launch ended after its first level
 };
 bool            resident_fits(dgraph const& g);
+// one block, one launch, for graphs that fit one SM's shared memory (small.cu)
+struct small_result
+{
+  uint64_t edges;                                    // adjacency entries read
+  uint32_t bad;                                      // validate_check's fault bits: nothing was computed
+  uint32_t trim_first, fwbw, trim, rest, rounds;     // vertices decided per phase; label rounds
+  uint32_t pivot, levels_fw, levels_bw;
+};
+constexpr size_t SMALL_RESULT_AT = 2048; // in kspn_context::h_state
+bool small_fits(dgraph const& g);
+void scc_small_async(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, small_result* res); // res: pinned host memory, complete with the stream
 void            fw_bw_trim_async(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, kspn_options const& opt, kspn_stats* st, cudaEvent_t after_kernel);
 resident_result fw_bw_trim_result(kspn_context* ctx, dgraph const& g, kspn_options const& opt, kspn_stats* st);
 // FW-BW from `pivot` and the trim-1 fixpoint of the remainder in one
