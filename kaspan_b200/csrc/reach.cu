@@ -1599,7 +1599,133 @@ struct joint_save
   unsigned long long barriers; // grid barriers the handing-off launch completed (the drop_barrier test hook counts on)
 };
 
-template<int MINB>
+// The searches' first levels while both are thin (at most THIN_E row entries
+// each), in block 0 alone: the other blocks wait at one barrier.  A grid-wide
+// level costs 12 us whatever it holds (a barrier and about eight dependent
+// accesses: tile, queue, offsets, neighbour, bitmap, its offsets, counter,
+// barrier); here the frontier stays in shared memory with its offsets, and a
+// level is four (neighbour, bitmap, offsets, block barrier), THIN_E
+// entries per direction side by side: half of the block's threads each.  Ends
+// after ASYNC_SLOW levels, when a search widens, runs dry or turns bottom-up;
+// the frontiers, scanned, and the control are left as a grid-wide level's.
+// Per level 12-13 -> 2.5-3.5 us; the frontiers' way back to the grid costs
+// about 6 once.  Whole call: G(n, m) n 65,536, degree 8: 189 -> 177 us;
+// n 3 M, degree 1.5: 1,169 -> 1,094; n 200,000, degree 3: 402 -> 376; random
+// geometric graph n 50,000: 954 -> 889.
+constexpr uint32_t THIN_E   = 512;
+constexpr int      THIN_ILP = THIN_E / (R_THREADS / 2);
+static_assert(4 * THIN_E * sizeof(unsigned long long) <= (EX_TILE + BU_BUF) * sizeof(uint32_t) && 2 * THIN_E <= 512 * 3, "the thin frontiers must fit the warp buffers");
+
+__device__ __forceinline__ bool
+thin_level(fwbw_args const& a, uint32_t lvl, uint64_t e0, uint64_t e1, unsigned long long m_u0, unsigned long long m_u1)
+{
+  return lvl < ASYNC_SLOW && lvl < a.cap && e0 <= THIN_E && e1 <= THIN_E && e0 <= m_u0 && e1 <= m_u1 && e0 * a.alpha <= m_u0 && e1 * a.alpha <= m_u1;
+}
+
+__device__ __noinline__ void
+thin_opening(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und)
+{
+  // per level (in turn) and direction: entries << 11 | vertices appended (a
+  // row counts THIN_E + 1 entries at most, and then sets s_long)
+  __shared__ uint32_t       s_next[3][2], s_long[2];
+  unsigned long long* const row = reinterpret_cast<unsigned long long*>(sm.warp);                // [parity][direction]: first entry << 24 | entries before it
+  uint32_t* const           ids = reinterpret_cast<uint32_t*>(sm.warp) + EX_TILE + BU_BUF; // [direction], of the newest level
+  int const                 d   = threadIdx.x >= R_THREADS / 2;
+  uint32_t const            tid = threadIdx.x & (R_THREADS / 2 - 1);
+  jdir const                D   = joint_dir(a, d);
+  uint32_t                  e[2], q[2] = { 1, 1 }, seen[2] = { 1, 1 }, rows = 0;
+  unsigned long long        m_u[2] = { a.m, a.m };
+  for (int i = 0; i < 2; ++i) e[i] = static_cast<uint32_t>(s_j.c[i] >> a.qbits);
+  if (tid == 0) row[d * THIN_E] = D.td_head[pivot] << 24, s_long[d] = 0, s_next[0][d] = s_next[1][d] = s_next[2][d] = 0;
+  __syncthreads();
+  uint32_t lvl = 0;
+  do {
+    unsigned long long const* const cur = row + ((lvl & 1u) * 2 + d) * THIN_E;
+    unsigned long long* const       nxt = row + (((lvl + 1) & 1u) * 2 + d) * THIN_E;
+    uint32_t* const                 ctr = s_next[lvl % 3];
+    uint32_t const                  ne = e[d], nq = q[d];
+    uint32_t                        w[THIN_ILP], took = 0;
+    uint64_t                        b[THIN_ILP], len[THIN_ILP];
+#pragma unroll
+    for (int k = 0; k < THIN_ILP; ++k) {
+      uint32_t const x = tid + k * (R_THREADS / 2);
+      w[k]             = pivot;
+      if (x < ne) {
+        uint32_t j = 0; // the last row that starts at or before entry x
+        for (uint32_t step = nq > 1 ? 1u << (31 - __clz(nq - 1)) : 0u; step; step >>= 1)
+          if (j + step < nq && (cur[j + step] & 0xFFFFFFu) <= x) j += step;
+        w[k] = D.td_adj[(cur[j] >> 24) + (x - static_cast<uint32_t>(cur[j] & 0xFFFFFFu))];
+      }
+    }
+    // the offsets are fetched beside the claim, for entries in vain too
+#pragma unroll
+    for (int k = 0; k < THIN_ILP; ++k) {
+      if (tid + k * (R_THREADS / 2) >= ne) continue;
+      b[k] = D.td_head[w[k]], len[k] = D.td_head[w[k] + 1];
+      if (bit_take(D.avail, w[k])) took |= 1u << k;
+    }
+#pragma unroll
+    for (int k = 0; k < THIN_ILP; ++k)
+      if ((took >> k) & 1u) {
+        bit_claim(D.mark, w[k]);
+        len[k] -= b[k];
+        if (len[k] > THIN_E) len[k] = THIN_E + 1, s_long[d] = 1;
+        uint32_t const old = atomicAdd(ctr + d, static_cast<uint32_t>(len[k]) << 11 | 1u);
+        uint32_t const at  = old & 0x7FFu;
+        nxt[at]            = b[k] << 24 | old >> 11;
+        ids[d * THIN_E + at] = w[k];
+      }
+    __syncthreads();
+    stamp(a, 4u);
+    if (threadIdx.x < 2) s_next[(lvl + 2) % 3][threadIdx.x] = 0;
+    for (int i = 0; i < 2; ++i) {
+      m_u[i] -= e[i];
+      rows += q[i];
+      q[i] = ctr[i] & 0x7FFu, e[i] = ctr[i] >> 11;
+      seen[i] += q[i];
+    }
+    ++lvl;
+  } while (q[0] && q[1] && thin_level(a, lvl, e[0], e[1], m_u[0], m_u[1]));
+  // the newest frontiers, scanned; one with a long row by way of the block queue
+  unsigned long long const* const last = row + ((lvl & 1u) * 2 + d) * THIN_E;
+  bool const                      long0 = s_long[0] != 0, long1 = s_long[1] != 0;
+  if (!(d ? long1 : long0)) {
+    frontier_buf const F = jbuf(D, lvl);
+    for (uint32_t k = tid; k < q[d]; k += R_THREADS / 2) {
+      uint32_t const pre = static_cast<uint32_t>(last[k] & 0xFFFFFFu), end = k + 1 < q[d] ? static_cast<uint32_t>(last[k + 1] & 0xFFFFFFu) : e[d];
+      F.q[k]      = ids[d * THIN_E + k];
+      F.prefix[k] = pre;
+      put_tile_starts(F.tile_start, pre, end - pre, k, a.m);
+    }
+  }
+  unsigned long long c[2];
+  for (int i = 0; i < 2; ++i) {
+    c[i] = static_cast<unsigned long long>(e[i]) << a.qbits | q[i];
+    if (!(i ? long1 : long0)) continue;
+    jdir const F = joint_dir(a, i);
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < q[i]; k += R_THREADS) sm.buf()[k] = ids[i * THIN_E + k];
+    if (threadIdx.x == 0) sm.buf_n = q[i];
+    flush_scanned(sm, jbuf(F, lvl), &F.lq[lvl % 3], a.qbits, F.td_head, a.n, a.m);
+    c[i] = __ldcg(&F.lq[lvl % 3]);
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      s_j.c[i] = c[i];
+      s_j.lvl[i] = lvl;
+      s_j.edges_td[i] = a.m - m_u[i];
+      s_j.m_u[i]      = m_u[i];
+      s_j.seen[i]     = seen[i];
+    }
+    a.st->rows_td += rows, a.st->pushed_td += seen[0] + seen[1] - 2;
+    auto* const js = static_cast<joint_save*>(a.jsave);
+    js->j          = s_j;
+    js->glvl       = lvl;
+    js->n_und      = n_und;
+  }
+}
+
+template<int MINB, bool THIN>
 __device__ __forceinline__ int
 run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uint32_t& glvl, unsigned long long& epoch, bool resume)
 {
@@ -1625,6 +1751,17 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
       s_j.restrict_to[d]                                               = 0;
     }
     if (!resume) s_j.capped = 0, s_j.seeded = 0;
+  }
+  if constexpr (THIN) {
+    __syncthreads();
+    // (the barrier hook belongs to grid-wide levels)
+    if (!a.drop_barrier && a.m >> 40 == 0 && thin_level(a, 0, s_j.c[0] >> a.qbits, s_j.c[1] >> a.qbits, a.m, a.m)) {
+      if (blockIdx.x == 0) thin_opening(a, sm, pivot, n_und);
+      if (!gsync(a, epoch)) return SEARCH_FAILED;
+      auto const* const js = static_cast<joint_save const*>(a.jsave);
+      if (threadIdx.x == 0 && blockIdx.x) s_j = js->j;
+      glvl = __ldcg(&js->glvl);
+    }
   }
   int  rc         = SEARCH_DONE;
   bool resume_now = resume; // the first iteration of a resume launch starts at its worklist phase
@@ -2398,9 +2535,12 @@ write_ids(fwbw_args const& a, uint32_t words, bool search, uint32_t scc)
 // keep their loads in flight without spills: with several start vertices
 // the phase has work for every warp (RGG 2^24, whole call: 2 blocks 6.44 ms,
 // 3: 5.73, 4: 5.37 but slower on shorter phases).
-template<int MINB>
+// THIN: with the thin opening.  A launch of its own for the pivot model, which
+// scores the pivot during a grid-wide first level: the opening's call costs
+// the levels' code 40 bytes of spills (R-MAT scale 26: 1,221 -> 1,233 us).
+template<int MINB, bool THIN>
 __global__ void __launch_bounds__(R_THREADS, MINB)
-k_fwbw(fwbw_args a)
+k_fwbw(fwbw_args const __grid_constant__ a)
 {
   __shared__ fwbw_smem sm;
   if (a.gate && __ldcg(a.gate)) return; // the same word for every block
@@ -2475,7 +2615,7 @@ k_fwbw(fwbw_args a)
     }
   }
   if (search) {
-    if (rc == SEARCH_DONE) rc = run_joint<MINB>(a, sm, p, n_und, glvl, epoch, a.resume != 0);
+    if (rc == SEARCH_DONE) rc = run_joint<MINB, THIN>(a, sm, p, n_und, glvl, epoch, a.resume != 0);
     if (rc == SEARCH_DONE && a.min_ids) {
       // smallest member = first set bit of vis_a & vis_b.  Every block first looks
       // at the same leading MIN_WORDS words (the SCC is usually dense
@@ -2725,7 +2865,7 @@ fwbw_grid(kspn_context* ctx)
 {
   if (!ctx->search_grid) {
     int bps = 0, sms = 0;
-    KSPN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_fwbw<4>, R_THREADS, 0));
+    KSPN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_fwbw<4, true>, R_THREADS, 0));
     KSPN_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     if (bps < 1) throw error{ KSPN_ERR_CUDA, "persistent FW-BW kernel does not fit on an SM" };
     // at most AW_GRID_MAX blocks: the worklist's spare slots (AW_STALE)
@@ -2751,7 +2891,7 @@ resume_grid(kspn_context* ctx)
 {
   if (!ctx->resume_grid) {
     int bps = 0, sms = 0;
-    KSPN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_fwbw<3>, R_THREADS, 0));
+    KSPN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_fwbw<3, false>, R_THREADS, 0));
     KSPN_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     if (bps < 1) throw error{ KSPN_ERR_CUDA, "persistent FW-BW resume kernel does not fit on an SM" };
     ctx->resume_grid = static_cast<unsigned>(std::min<int>(bps * sms, AW_GRID_MAX));
@@ -2858,7 +2998,8 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
   ctx->fwbw_after = after_kernel;
   void* args[]    = { &a };
   barrier_for_grid(ctx, fwbw_grid(ctx));
-  KSPN_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(&k_fwbw<4>), dim3(fwbw_grid(ctx)), dim3(R_THREADS), args, 0, ctx->stream));
+  auto* const kernel = a.model ? reinterpret_cast<void const*>(&k_fwbw<4, false>) : reinterpret_cast<void const*>(&k_fwbw<4, true>);
+  KSPN_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(fwbw_grid(ctx)), dim3(R_THREADS), args, 0, ctx->stream));
   ctx->launches += 1;
   if (after_kernel) KSPN_CUDA(cudaEventRecord(after_kernel, ctx->stream));
   // results, and the barrier's error word (read after the launch ended: a
@@ -2885,7 +3026,7 @@ check_persistent(kspn_context* ctx)
     a.resume     = 1;
     void* args[] = { &a };
     barrier_for_grid(ctx, resume_grid(ctx));
-    KSPN_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(&k_fwbw<3>), dim3(resume_grid(ctx)), dim3(R_THREADS), args, 0, ctx->stream));
+    KSPN_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(&k_fwbw<3, false>), dim3(resume_grid(ctx)), dim3(R_THREADS), args, 0, ctx->stream));
     ctx->launches += 1;
     if (ctx->fwbw_after) KSPN_CUDA(cudaEventRecord(ctx->fwbw_after, ctx->stream));
     KSPN_CUDA(cudaMemcpyAsync(hs, ctx->ws.rstate, sizeof(reach_state), cudaMemcpyDeviceToHost, ctx->stream));
