@@ -2093,11 +2093,15 @@ __device__ __forceinline__ uint32_t
 count_live(uint32_t const* snap, uint32_t const* __restrict__ adj, uint64_t b, uint64_t e)
 {
   uint32_t c = 0;
-  for (; b + 4 <= e; b += 4) {
-    uint32_t const x0 = adj[b], x1 = adj[b + 1], x2 = adj[b + 2], x3 = adj[b + 3];
-    c += snap_bit(snap, x0) + snap_bit(snap, x1) + snap_bit(snap, x2) + snap_bit(snap, x3);
+  for (; b < e; b += 4) {
+    uint32_t x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[k] = adj[b + k < e ? b + k : b];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[k] = snap_bit(snap, x[k]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c += b + k < e ? x[k] : 0u;
   }
-  for (; b < e; ++b) c += snap_bit(snap, adj[b]);
   return c;
 }
 
@@ -2196,55 +2200,66 @@ trim_push(fwbw_args const& a, uint32_t const* qin, uint32_t qn, uint32_t* qout, 
       warp_push_active64(w, qout, octr, a.n);
     }
   };
-  // a lane's own row: four neighbour ids, then their four und words, in
-  // flight at once
+  // a lane's own row, four neighbours at a time (the last step's short ones
+  // too): their ids, then their und words, then their decrements in flight
+  // at once
   auto const row = [&](uint32_t const* adj, uint64_t b, uint64_t e, uint32_t* deg) {
-    for (; b + 4 <= e; b += 4) {
-      uint32_t w[4], u[4];
+    for (; b < e; b += 4) {
+      uint32_t w[4], old[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) w[k] = adj[b + k];
+      for (int k = 0; k < 4; ++k) w[k] = adj[b + k < e ? b + k : b];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) u[k] = __ldcg(a.und + (w[k] >> 5));
+      for (int k = 0; k < 4; ++k) old[k] = __ldcg(a.und + (w[k] >> 5));
 #pragma unroll
-      for (int k = 0; k < 4; ++k) hit(w[k], u[k], deg);
-    }
-    for (; b < e; ++b) {
-      uint32_t const w = adj[b];
-      hit(w, __ldcg(a.und + (w >> 5)), deg);
+      for (int k = 0; k < 4; ++k) old[k] = b + k < e && ((old[k] >> (w[k] & 31)) & 1u) ? atomicSub(deg + w[k], 1u) : 0u;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (old[k] == 1u && bit_take(a.und, w[k])) {
+          if (!a.ids_at_end) a.scc_id[w[k]] = w[k];
+          ++dec;
+          warp_push_active64(w[k], qout, octr, a.n);
+        }
     }
   };
+  // a queued vertex's two rows are walked by different threads
+  for (uint64_t t2 = static_cast<uint64_t>(blockIdx.x) * R_THREADS + threadIdx.x; t2 < 2 * span; t2 += static_cast<uint64_t>(gridDim.x) * R_THREADS) {
+    bool const      dir  = t2 >= span;
+    uint64_t const* head = dir ? a.bh : a.fh;
+    uint32_t const* adj  = dir ? a.bc : a.fc;
+    uint32_t*       deg  = dir ? a.outdeg : a.indeg;
+    uint64_t const  t    = dir ? t2 - span : t2;
+    bool const     have = t < qn;
+    uint32_t const u    = have ? __ldcg(qin + t) : 0u;
+    uint64_t       b = 0, e = 0;
+    if (have) b = head[u], e = head[u + 1];
+    bool const big = have && e - b >= TRIM_SMALL;
+    edges += e - b;
+    if (have && !big) row(adj, b, e, deg);
+    for (unsigned todo = __ballot_sync(0xFFFFFFFFu, big); todo; todo &= todo - 1) {
+      unsigned const l  = __ffs(todo) - 1;
+      uint64_t const b0 = __shfl_sync(0xFFFFFFFFu, b, l), e0 = __shfl_sync(0xFFFFFFFFu, e, l);
+      if (e0 - b0 > HEAVY_ROW) {
+        // listed for the next level's slices (front: out-rows, back:
+        // in-rows; they never meet, heavy_capacity covers both)
+        if (lane == l) {
+          uint32_t const i = atomicAdd(hout.n + dir, 1u);
+          if (i < a.heavy_cap / 2) hout.list[dir ? a.heavy_cap - 1 - i : i] = u;
+          else atomicExch(&a.st->heavy_err, 1u);
+        }
+        continue;
+      }
+      for (uint64_t x = b0 + lane; x < e0; x += 32) {
+        uint32_t const w = adj[x];
+        hit(w, __ldcg(a.und + (w >> 5)), deg);
+      }
+    }
+  }
+  // rows the last level left to slices
 #pragma unroll 1
   for (int dir = 0; dir < 2; ++dir) {
     uint64_t const* head = dir ? a.bh : a.fh;
     uint32_t const* adj  = dir ? a.bc : a.fc;
     uint32_t*       deg  = dir ? a.outdeg : a.indeg;
-    for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * R_THREADS + threadIdx.x; t < span; t += static_cast<uint64_t>(gridDim.x) * R_THREADS) {
-      bool const     have = t < qn;
-      uint32_t const u    = have ? __ldcg(qin + t) : 0u;
-      uint64_t       b = 0, e = 0;
-      if (have) b = head[u], e = head[u + 1];
-      bool const big = have && e - b >= TRIM_SMALL;
-      edges += e - b;
-      if (have && !big) row(adj, b, e, deg);
-      for (unsigned todo = __ballot_sync(0xFFFFFFFFu, big); todo; todo &= todo - 1) {
-        unsigned const l  = __ffs(todo) - 1;
-        uint64_t const b0 = __shfl_sync(0xFFFFFFFFu, b, l), e0 = __shfl_sync(0xFFFFFFFFu, e, l);
-        if (e0 - b0 > HEAVY_ROW) {
-          // listed for the next level's slices (front: out-rows, back:
-          // in-rows; they never meet, heavy_capacity covers both)
-          if (lane == l) {
-            uint32_t const i = atomicAdd(hout.n + dir, 1u);
-            if (i < a.heavy_cap / 2) hout.list[dir ? a.heavy_cap - 1 - i : i] = u;
-            else atomicExch(&a.st->heavy_err, 1u);
-          }
-          continue;
-        }
-        for (uint64_t x = b0 + lane; x < e0; x += 32) {
-          uint32_t const w = adj[x];
-          hit(w, __ldcg(a.und + (w >> 5)), deg);
-        }
-      }
-    }
     uint32_t const hn = dir ? hn1 : hn0;
     heavy_slices(dir ? hin.list + a.heavy_cap - hn : hin.list, hn, head, [&](uint32_t, uint32_t, uint64_t b0, uint64_t e0) {
       for (uint64_t x = b0 + lane; x < e0; x += 32) {
