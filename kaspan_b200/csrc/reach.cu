@@ -2096,11 +2096,13 @@ count_live(uint32_t const* snap, uint32_t const* __restrict__ adj, uint64_t b, u
   for (; b < e; b += 4) {
     uint32_t x[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) x[k] = adj[b + k < e ? b + k : b];
+    for (int k = 0; k < 4; ++k)
+      if (x[k] = 0; b + k < e) x[k] = adj[b + k];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) x[k] = snap_bit(snap, x[k]);
+    for (int k = 0; k < 4; ++k)
+      if (b + k < e) x[k] = snap_bit(snap, x[k]);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) c += b + k < e ? x[k] : 0u;
+    for (int k = 0; k < 4; ++k) c += x[k];
   }
   return c;
 }
@@ -2207,11 +2209,13 @@ trim_push(fwbw_args const& a, uint32_t const* qin, uint32_t qn, uint32_t* qout, 
     for (; b < e; b += 4) {
       uint32_t w[4], old[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) w[k] = adj[b + k < e ? b + k : b];
+      for (int k = 0; k < 4; ++k)
+        if (w[k] = 0; b + k < e) w[k] = adj[b + k];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) old[k] = __ldcg(a.und + (w[k] >> 5));
+      for (int k = 0; k < 4; ++k)
+        if (old[k] = 0; b + k < e) old[k] = __ldcg(a.und + (w[k] >> 5));
 #pragma unroll
-      for (int k = 0; k < 4; ++k) old[k] = b + k < e && ((old[k] >> (w[k] & 31)) & 1u) ? atomicSub(deg + w[k], 1u) : 0u;
+      for (int k = 0; k < 4; ++k) old[k] = (old[k] >> (w[k] & 31)) & 1u ? atomicSub(deg + w[k], 1u) : 0u;
 #pragma unroll
       for (int k = 0; k < 4; ++k)
         if (old[k] == 1u && bit_take(a.und, w[k])) {
