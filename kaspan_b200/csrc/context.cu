@@ -286,9 +286,11 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
     ~prof_reset() { c->prof = nullptr; }
   } prof_guard{ ctx };
   cudaEvent_t t_begin = ctx->ev[KSPN_PHASES], t_end = ctx->ev[KSPN_PHASES + 1];
-  KSPN_CUDA(cudaEventRecord(t_begin, ctx->stream));
+  // events time the phases of a call that asked for statistics; without it
+  // the host waits for the stream (each record is host time before the next launch)
+  if (st) KSPN_CUDA(cudaEventRecord(t_begin, ctx->stream));
   phase_clock clk{ ctx, st };
-  clk.start();
+  if (st) clk.start();
   // the resident pipeline queues the checks ahead of its launches, which
   // leave the graph's rows alone when a fault bit is set, and reads the bits
   // with its results: no host round trip of their own
@@ -414,20 +416,22 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
       // trim_1_first, then FW-BW and the trim fixpoint in ONE persistent
       // launch that takes the pivot from device memory: one host sync
       trim_1_first_async(ctx, g, und, opt.validate != 0);
-      KSPN_CUDA(cudaEventRecord(ctx->ev[2], ctx->stream));
+      if (st) KSPN_CUDA(cudaEventRecord(ctx->ev[2], ctx->stream));
+      auto const finished = [&] { // (ev[3]: the phase clock's end)
+        if (st) KSPN_CUDA(cudaEventRecord(ctx->ev[3], ctx->stream));
+        KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
+      };
       // with the learned rule the launch first scores the plain pivot (no
       // extra launch when the model accepts it)
-      fw_bw_trim_async(ctx, g, und, scc_id, opt, st, ctx->ev[4]);
+      fw_bw_trim_async(ctx, g, und, scc_id, opt, st, st ? ctx->ev[4] : nullptr);
       KSPN_CUDA(cudaMemcpyAsync(ctx->h_ctr, ws.ctr, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-      KSPN_CUDA(cudaEventRecord(ctx->ev[3], ctx->stream));
-      KSPN_CUDA(cudaEventSynchronize(ctx->ev[3]));
+      finished();
       look_back_check(ctx);
       if (opt.validate) validate_check(ctx->h_ctr[CTR_ERR]);
       resident_result r = fw_bw_trim_result(ctx, g, opt, st);
       if (r.resumed) {
         // the phase clock's end after the resume launch
-        KSPN_CUDA(cudaEventRecord(ctx->ev[3], ctx->stream));
-        KSPN_CUDA(cudaEventSynchronize(ctx->ev[3]));
+        finished();
       }
       if (r.pivot_rejected) {
         // the model rejected the plain pivot: score every candidate, then
@@ -435,13 +439,11 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
         learned_pivot(ctx, g, ctx->pivot_model, false);
         kspn_options o2  = opt;
         o2.learned_pivot = 0;
-        fw_bw_trim_async(ctx, g, und, scc_id, o2, st, ctx->ev[4]);
-        KSPN_CUDA(cudaEventRecord(ctx->ev[3], ctx->stream));
-        KSPN_CUDA(cudaEventSynchronize(ctx->ev[3]));
+        fw_bw_trim_async(ctx, g, und, scc_id, o2, st, st ? ctx->ev[4] : nullptr);
+        finished();
         r = fw_bw_trim_result(ctx, g, opt, st);
         if (r.resumed) {
-          KSPN_CUDA(cudaEventRecord(ctx->ev[3], ctx->stream));
-          KSPN_CUDA(cudaEventSynchronize(ctx->ev[3]));
+          finished();
         }
       }
       uint32_t const        tf = ctx->h_ctr[CTR_DECIDED];
@@ -512,19 +514,19 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
   // (id = smallest member) already name components canonically; label
   // searches name them after their root, so only then is a relabel needed
   if (und_checked) {
-    // everything was decided by the resident launch, whose completion
-    // event (now ev[0]) the host already waited for: no further sync
+    // everything was decided by the resident launch, for which the host has
+    // already waited (with st, its event is now ev[0]): no further sync
     t_end = ctx->ev[0];
   } else {
     // und is counted on the way: the count comes back with the relabel's
     // check, or alone
     count_undecided_async(ctx, g.n, und);
     if (label_ran) canonicalise(ctx, g.n, scc_id, ws.label, true);
-    KSPN_CUDA(cudaEventRecord(t_end, ctx->stream));
+    if (st) KSPN_CUDA(cudaEventRecord(t_end, ctx->stream));
     if (!label_ran) read_counters(ctx);
     if (ctx->h_ctr[CTR_LEFT]) throw error{ KSPN_ERR_INTERNAL, "decided-vertex count does not match n" };
     add(KSPN_PHASE_CANON, 0);
-    KSPN_CUDA(cudaEventSynchronize(t_end));
+    if (st) KSPN_CUDA(cudaEventSynchronize(t_end)); // (the counters' read waited for the stream)
   }
   if (st) st->edges_scanned = ctx->h_ctr64[0] + ctx->td_edges;
   if (st) {
