@@ -412,7 +412,8 @@ struct kspn_context
   kspn_stats*        prof       = nullptr;
   cudaEvent_t        pe[4]      = {};
   void*              h_state    = nullptr; // pinned 4 KiB: mirror of ws.rstate, trim state at 512, small_result at SMALL_RESULT_AT, look-back fault word last
-  unsigned           search_grid = 0;      // blocks of the persistent FW-BW launch
+  unsigned           search_grid = 0;      // most blocks of the persistent FW-BW launch that are resident at once
+  unsigned           search_sms  = 0;
   unsigned           resume_grid = 0;      // blocks of its resume launch (the worklist phase)
   unsigned           bar_grid    = 0;      // grid of the last launch on the workspace's grid barrier
   bool               union_route = false;  // the pipeline runs on a batch mix as one graph: no second FW-BW
