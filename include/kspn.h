@@ -375,7 +375,7 @@ int kspn_mlp_adam(kspn_context* ctx, float* d_params, const float* d_grad, float
  * (fw) and CSC (bw) over n_total = vtx_off[count] vertices: heads hold
  * global edge positions, rows hold LOCAL ids (0 .. n_g - 1).  Output:
  * scc_id[vtx_off[g] + v] = the local id of the smallest member of v's SCC.
- * Graphs of at most 512 vertices and 2048 edges are decomposed by one warp
+ * Graphs of at most 32 vertices and 2048 edges are decomposed by one warp
  * each (Tarjan in shared memory), larger ones by one block or, from
  * n + m >= cluster_min, one thread-block cluster each (trim-1, FW-BW
  * rounds, Tarjan of the remainder), all in one captured CUDA graph
@@ -385,7 +385,8 @@ int kspn_mlp_adam(kspn_context* ctx, float* d_params, const float* d_grad, float
 typedef struct kspn_batch_options {
     uint32_t max_rounds;   /* FW-BW rounds per large graph before one thread's Tarjan finishes it (0: 64) */
     uint32_t rem_tarjan;   /* a large graph's remainder of at most this many vertices goes to the
-                              shared-memory Tarjan (0: 512, the most it holds) */
+                              shared-memory Tarjan (0: 512, the most it holds); before its first
+                              FW-BW round only one of at most 64 */
     uint32_t cluster_size; /* blocks of the thread-block cluster a large graph gets (1..8; 0: 1, a block) */
     uint32_t reserved0;
     uint64_t cluster_min;  /* with cluster_size > 1: n + m from which a graph gets a cluster

@@ -10,7 +10,7 @@
 // member of v's SCC.
 //
 // Plan (device, captured): per graph its size class -- a graph of at most
-// RS_MAXV vertices and RS_MAXE edges is "small" -- and its bitmap word
+// BT_WARP_N vertices and RS_MAXE edges is "small" -- and its bitmap word
 // offset (each graph owns whole bitmap words); the large graphs sorted by
 // n + m, largest first (a work queue in that order balances the tail).
 // Solve (kernels on parallel branches of the same CUDA graph, so they
@@ -21,9 +21,9 @@
 //    memory (up to 2^18 vertices, two block sizes): init (degrees, in/out = 0
 //    decided), then rounds of {trim-1 push levels, FW-BW from the largest
 //    in*out (SCC named by its smallest member), live degrees recounted} until
-//    the remainder has at most `rem_tarjan` vertices -- then Tarjan in shared
-//    memory -- or the round cap is reached -- then one thread's Tarjan in
-//    global memory;
+//    the remainder has at most `rem_tarjan` vertices (64 before the first
+//    FW-BW) -- then Tarjan in shared memory -- or the round cap is reached --
+//    then one thread's Tarjan in global memory;
 //  * k_batch_group: the same rounds with bitmaps in global memory, for larger
 //    graphs, the joint searches (option search = 1) and thread-block clusters
 //    (up to 8 blocks, distributed shared memory, the cluster barrier) for
@@ -73,6 +73,7 @@ struct bt_args
   uint32_t        joint;      // FW and BW searches at the same time (bt_reach_joint)
 };
 
+constexpr uint32_t BT_WARP_N = 32; // vertices up to which a warp's Tarjan solves a graph (2500 graphs of 2^6 .. 2^9: 0.26 ms; 64: 0.28, 128: 0.32, 512: 0.59)
 constexpr uint32_t BT_COUNT = 16, BT_CLAIM = 24;
 
 // How a graph is solved (the work queue's classes, in queue order).
@@ -111,7 +112,7 @@ k_bt_classify(uint32_t G, uint64_t const* __restrict__ vtx_off, uint64_t const* 
     uint64_t const vo = vtx_off[g], n = vtx_off[g + 1] - vo;
     uint64_t const m  = fh[vo + n] - fh[vo];
     uint64_t const size  = n + m;
-    uint32_t const cls   = n <= RS_MAXV && m <= RS_MAXE ? BT_WARP : (size >= cluster_min ? BT_CLUSTER : (joint || n > l_max || m >= 0xFFFFFFFFull ? BT_GLOBAL : (n > m_max ? BT_BLOCK_L : BT_BLOCK_M)));
+    uint32_t const cls   = n <= BT_WARP_N && m <= RS_MAXE ? BT_WARP : (size >= cluster_min ? BT_CLUSTER : (joint || n > l_max || m >= 0xFFFFFFFFull ? BT_GLOBAL : (n > m_max ? BT_BLOCK_L : BT_BLOCK_M)));
     keys[g]  = (cls << 29) | (0x1FFFFFFFu - static_cast<uint32_t>(size < 0x1FFFFFFFull ? size : 0x1FFFFFFFull));
     vals[g]  = g;
     words[g] = static_cast<uint32_t>((n + 31) / 32);
@@ -747,24 +748,36 @@ bt_solve(bt_args const& a, uint32_t gi, bt_group const& g, rs_piece& piece)
 // SCC member's rows being walked.
 // Every id is its vertex's own from the start (trimmed vertices keep it);
 // only SCC members are written again, from the bitmap.
-// Two sizes: BB_L (up to BB_L_WORDS bitmap words: 2^18 vertices, 96 KB, two
-// blocks of BB_L_THREADS per SM) and BB_M (2^16 vertices, 24 KB, four blocks
-// of BB_M_THREADS).
+// Two sizes: BB_L (up to BB_L_WORDS bitmap words: 2^18 vertices, 96 KB, one
+// block of BB_L_THREADS per SM) and BB_M (2^15 vertices, four blocks of
+// BB_M_THREADS).  With at most two graphs per SM every graph above BB_M_FEW
+// vertices gets the larger block: no other graph waits for the threads, and
+// the slowest graph is the call's time (120 graphs of 2^8 .. 2^16 vertices:
+// 0.69 -> 0.50 ms, 30 of 2^10 .. 2^13: 0.35 -> 0.32).
 // Measured on the 4096-graph mix (157 M vertices, 533 M edges): 17.1 ms with
 // bitmaps in global memory (k_batch_group), 14.3 with 1536 threads of 40
-// registers per SM (spills), 11.0 as it is: 10.9 to 11.2 over 2 to 4
-// neighbours at once, 2 or 3 vertices per round, 640 + 320 threads, BB_M up
-// to 2^17 vertices (11.5); 13.7 with blocks of 128.  DRAM traffic of the
-// graphs over 2^16 vertices: 31.3 -> 19.7 GB per 85 M vertices; it stays
-// latency-bound (2.4 TB/s).  Not kept: prefetching a find's offsets into L2
-// (12.1 ms), walking the SCC members' rows instead of the recount (+3%).
+// registers per SM (spills), 10.8 with two BB_L blocks of 512 threads, 8.5
+// with one of 1024 (half the graphs in flight leave each twice the L1 and
+// L2; 296 graphs of 2^17 and 2^18 vertices: 6.7 -> 4.3, 120 of 2^18: 6.7 ->
+// 2.9).  The line between the two at 2^16, 2^15, 2^14, 2^13: 8.50, 8.53,
+// 8.77, 9.00; 2000 graphs of 2^10 .. 2^15: 1.45, 1.46, 1.58, 1.76; 16 graphs
+// of 2^16: 1.37 at the first, 0.82 otherwise; BB_M of 512 threads: 8.86.
+// Not kept: prefetching a find's offsets into L2 (+10%), walking the SCC
+// members' rows instead of the recount (+3%), 4 neighbours at once (+1%), 1
+// or 4 vertices per round (+12%, +2%).
 constexpr int      BB_ILP       = 2; // neighbours of a row a lane reads at once
 constexpr int      BB_CAND      = 2; // vertices a lane takes per round of a pass in id order
-constexpr int      BB_L_THREADS = 512, BB_M_THREADS = 256;
-constexpr int      BB_L_BLOCKS = 2, BB_M_BLOCKS = 4; // per SM: 1024 threads of 64 registers
-constexpr uint32_t BB_L_WORDS = 8192, BB_M_WORDS = 2048;
+constexpr int      BB_L_THREADS = 1024, BB_M_THREADS = 256;
+constexpr int      BB_L_BLOCKS = 1, BB_M_BLOCKS = 4; // per SM: 1024 threads of 64 registers either way
+constexpr uint32_t BB_L_WORDS = 8192, BB_M_WORDS = 1024;
 constexpr uint32_t BB_LONG   = 32; // neighbours a lane walks alone; longer rows go to the whole warp
-constexpr uint32_t BB_BU_DIV = 16; // bottom-up when the frontier holds more than 1/16 of the candidates (1/10, 1/20: the same within 2%; 1/5: +4%, 1/50: +6%)
+constexpr uint32_t BB_BU_DIV = 10; // bottom-up when the frontier holds more than 1/10 of the candidates (4096 graphs: 8.46 ms, 1/16 the same, 1/8 8.59, 1/5 9.02; 200 graphs: 1.82, 1/16 1.96)
+constexpr uint32_t BB_M_FEW = 512;
+// A remainder goes to one lane's Tarjan (0.25 us per vertex and edge) from
+// rem_tarjan on, but not a whole graph before its first FW-BW round: that
+// leaves little in most.  30 graphs of 2^6 .. 2^9 vertices: 0.48 -> 0.13 ms,
+// 2000 of 2^8 .. 2^11: 0.70 -> 0.37 (limit 32, 128: the same within 5%).
+constexpr uint32_t BB_TARJAN_0 = 64;
 constexpr uint32_t BB_DEG8   = 255;
 
 constexpr uint32_t BB_ROUND = 32 * BB_CAND;    // vertices a warp takes per round
@@ -1376,7 +1389,7 @@ bb_solve(bt_args const& a, uint32_t gi, bb_block& B, rs_piece& piece, uint32_t s
     rem -= done - before;
     if (threadIdx.x == 0) bt_phase(a, g, 1, t);
     if (rem == 0) break;
-    if (rem <= a.rem_tarjan) {
+    if (rem <= (round ? a.rem_tarjan : min(a.rem_tarjan, BB_TARJAN_0))) {
       if (bb_tarjan(a, G, B, piece)) {
         if (threadIdx.x == 0) bt_phase(a, g, 4, t);
         break;
@@ -1462,8 +1475,10 @@ bb_solve(bt_args const& a, uint32_t gi, bb_block& B, rs_piece& piece, uint32_t s
 
 // Persistent blocks over class `cls` of the queue.  Dynamic shared memory:
 // und | va, vb (or the Tarjan piece over them) | the warps' pack buffers.
+template<uint32_t WORDS>
+constexpr uint32_t bb_scratch = std::max<uint32_t>(2 * WORDS, (sizeof(rs_piece) + 3) / 4); // va and vb, or the piece
 template<int T, uint32_t WORDS>
-constexpr size_t bb_dyn_bytes = 3 * WORDS * sizeof(uint32_t) + T / 32 * BB_PACK * sizeof(uint16_t);
+constexpr size_t bb_dyn_bytes = (WORDS + bb_scratch<WORDS>) * sizeof(uint32_t) + T / 32 * BB_PACK * sizeof(uint16_t);
 
 template<int T, int BLOCKS, uint32_t WORDS>
 __global__ void __launch_bounds__(T, BLOCKS)
@@ -1471,14 +1486,13 @@ k_batch_block(bt_args a, uint32_t cls)
 {
   extern __shared__ __align__(16) uint32_t bb_dyn[];
   __shared__ bb_smem s;
-  static_assert(2 * WORDS * sizeof(uint32_t) >= sizeof(rs_piece), "the Tarjan piece must fit the two reach bitmaps");
   static_assert(WORDS / 8 / (T / 32) <= 256, "a packed vertex is 8 bits of group, 8 of place");
   bb_block B;
   B.S    = &s;
   B.und  = bb_dyn;
   B.va   = bb_dyn + WORDS;
   B.vb   = bb_dyn + 2 * WORDS;
-  B.pack = reinterpret_cast<uint16_t*>(bb_dyn + 3 * WORDS) + (threadIdx.x >> 5) * BB_PACK;
+  B.pack = reinterpret_cast<uint16_t*>(bb_dyn + WORDS + bb_scratch<WORDS>) + (threadIdx.x >> 5) * BB_PACK;
   uint32_t const first = bt_first(a.ctr, cls), count = __ldcg(a.ctr + BT_COUNT + cls);
   for (;;) {
     if (threadIdx.x == 0) s.claim = atomicAdd(a.ctr + BT_CLAIM + cls, 1u);
@@ -1628,7 +1642,7 @@ enqueue_batch(kspn_context* ctx, batch_cache& c, bt_args const& a0)
   uint32_t const     G = c.G;
   KSPN_CUDA(cudaMemsetAsync(p.ctr, 0, 64 * sizeof(uint32_t), s));
   unsigned const cgrid = div_up(G, 256);
-  k_bt_classify<<<cgrid < 1 ? 1 : cgrid, 256, 0, s>>>(G, a0.vtx_off, a0.fh, c.cluster_min, c.joint, BB_L_WORDS * 32, BB_M_WORDS * 32, p.keys, p.order, p.words, p.ctr);
+  k_bt_classify<<<cgrid < 1 ? 1 : cgrid, 256, 0, s>>>(G, a0.vtx_off, a0.fh, c.cluster_min, c.joint, BB_L_WORDS * 32, G <= 2 * c.l_blocks ? BB_M_FEW : BB_M_WORDS * 32, p.keys, p.order, p.words, p.ctr);
   KSPN_CHECK_LAUNCH();
   exclusive_scan<uint64_t>(s, f_words{ p.words }, G, p.word_off, p.part64, nullptr);
   radix_sort_pairs(ctx, p.keys, p.order, p.kalt, p.valt, G, 0, 32, p.hist);

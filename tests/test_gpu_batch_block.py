@@ -1,6 +1,5 @@
 """The batched path's classes at their edges: graphs just inside and outside
-the block sizes (2^16 and 2^18 vertices), the warp path (512 vertices, 2048
-edges), rows longer than a lane walks alone, degrees that need 32-bit counts,
+the block sizes (512 or 2^15, and 2^18 vertices), the warp path (32 vertices), rows longer than a lane walks alone, degrees that need 32-bit counts,
 and graphs whose rest after the first SCC is larger or smaller than it; each
 against the oracle's Tarjan."""
 import numpy as np
@@ -64,6 +63,14 @@ def run(ctx, graphs):
 def test_class_edges(ctx, degree):
     sizes = [1, 31, 32, 33, 511, 512, 513, 600, 1023, 2049, 8191, 16384, 65535, 65536, 65537, 131071, 262143, 262144, 262145]
     run(ctx, [gnm(n, degree, 3 * n) for n in sizes])
+
+
+@pytest.mark.parametrize("degree", [0.9, 1.6])
+def test_classes_of_large_counts(ctx, degree):
+    """More than two graphs per SM, where the larger block starts at 2^15
+    vertices instead of 512; remainders around the first round's 64."""
+    sizes = [32767, 32768, 32769, 511, 512, 513] + [20 + i % 60 for i in range(700)]
+    run(ctx, [gnm(n, degree, 5 * n + i) for i, n in enumerate(sizes)])
 
 
 @pytest.mark.parametrize("fan", [31, 33, 200, 254, 255, 256, 3000])
