@@ -1,4 +1,4 @@
-// Residual device finish: Tarjan on the undecided sub-graph.
+// Residual device finish: the undecided sub-graph, piece by piece.
 //
 // Reference: the residual step of variant/scc_trim_ex_residual.hpp:110-127
 // (also scc_ispan_like.hpp, scc_trim_ex_light_residual.hpp):
@@ -8,7 +8,7 @@
 // named by its smallest original vertex id.
 //
 // On the device the sub-graph splits into weakly connected pieces (an SCC
-// never spans two), and one warp decomposes each small piece:
+// never spans two), and one warp or block decomposes each small piece:
 //   1. the undecided vertices are listed (every later pass runs over the
 //      list), and union-find over their out-edges to undecided vertices joins
 //      them (hooking the larger root under the smaller with atomicCAS, path
@@ -20,15 +20,15 @@
 //   3. a piece of up to 32 vertices goes to a warp, lane = vertex: rows become
 //      bit masks, Warshall's closure takes one shuffle per vertex, and an SCC is
 //      the closure and its transpose (one ballot per vertex); a piece of up to
-//      RS_MAXV vertices and RS_MAXE internal edges goes to a warp's
-//      shared-memory Tarjan (lane 0, explicit stacks).  Either way each member
-//      gets its SCC's smallest vertex and leaves und.
+//      RS_MAXV vertices and RS_MAXE internal edges goes to a block, trim and
+//      label rounds in shared memory.  Either way each member gets its SCC's
+//      smallest vertex and leaves und.
 // Larger pieces stay undecided; the pipeline's label rounds finish them.
 // Bound: launches and the latency of a few dependent loads each.  RGG of 10^6
 // vertices (29,636 undecided, whole step): 390 us with ordered compaction,
-// a radix sort by root and every piece through Tarjan.
-#include "kspn_internal.cuh"
+// a radix sort by root and every piece through one lane's Tarjan.
 #include "prim.cuh"
+#include "small.cuh"
 #include "tarjan_smem.cuh"
 
 #include <algorithm>
@@ -38,7 +38,6 @@ namespace kspn {
 namespace {
 
 constexpr int      RS_THREADS = 256;
-constexpr int      RS_WARPS   = 4;    // warps per block of the Tarjan kernel
 constexpr uint32_t RS_FIND    = 1u << 20; // bound on one find / unite loop
 
 unsigned
@@ -308,94 +307,110 @@ k_res_small(rs_counts const* __restrict__ rc, uint32_t const* __restrict__ piece
   if (lane == 0 && dec) atomicAdd(decided, dec);
 }
 
-// One warp per piece of 33 to RS_MAXV vertices and at most RS_MAXE internal
-// edges; local index = place in the piece.
-__global__ void __launch_bounds__(RS_WARPS * 32)
-k_res_tarjan(rs_counts const* __restrict__ rc, uint32_t const* __restrict__ pieces, uint32_t cap, uint32_t const* __restrict__ count, uint32_t const* __restrict__ start,
-             uint32_t const* __restrict__ place, uint32_t const* __restrict__ members, uint64_t const* __restrict__ fh, uint32_t const* __restrict__ fc, uint32_t* und,
-             uint32_t* __restrict__ scc_id, uint32_t* decided, uint32_t* big)
+// One block per piece of 33 to RS_MAXV vertices and at most RS_MAXE internal
+// edges, in shared memory: local index = place in the piece, the rows of both
+// directions built from the out-rows' undecided neighbours, then trim and
+// label rounds (small.cuh).  One lane's Tarjan of such a piece took 0.25 us
+// per vertex and edge, 300 us and more for the largest; a level here takes
+// about 0.25 us.  Whole call, random geometric graphs of 250,000 / 10^6 / 4 M
+// vertices: 1,051 / 1,025 / 2,154 -> 919 / 933 / 1,887 us; 128 threads 934 /
+// 936 / 1,930, 512 threads the same within 2%.
+constexpr int RB_T = 256;
+struct rb_piece
 {
-  extern __shared__ __align__(16) unsigned char rs_smem[];
-  unsigned const  lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-  rs_piece&       p    = reinterpret_cast<rs_piece*>(rs_smem)[wid];
-  uint32_t const  S    = rc->mid;
-  uint32_t        dec  = 0;
-  for (uint32_t sgi = blockIdx.x * RS_WARPS + wid; sgi < S; sgi += gridDim.x * RS_WARPS) {
-    uint32_t const root = pieces[cap - 1 - sgi], k = count[root], b = start[root];
-    bool           heavy_row = false;
-    for (uint32_t i = lane; i < k; i += 32) {
+  uint32_t vid[RS_MAXV], edge[RS_MAXE], lab[RS_MAXV], out_at[RS_MAXV], in_at[RS_MAXV];
+  uint32_t und[RS_MAXV / 32], open[RS_MAXV / 32], vis[RS_MAXV / 32], inq[RS_MAXV / 32];
+  uint16_t q0[RS_MAXV], q1[RS_MAXV], fh[RS_MAXV + 2], bh[RS_MAXV + 2], fc[RS_MAXE], bc[RS_MAXE];
+  uint32_t edges;
+};
+
+__global__ void __launch_bounds__(RB_T)
+k_res_block(rs_counts const* __restrict__ rc, uint32_t const* __restrict__ pieces, uint32_t cap, uint32_t const* __restrict__ count, uint32_t const* __restrict__ start,
+            uint32_t const* __restrict__ place, uint32_t const* __restrict__ members, uint64_t const* __restrict__ fh, uint32_t const* __restrict__ fc, uint32_t* und,
+            uint32_t* scc_id, uint32_t* decided, uint32_t* big)
+{
+  __shared__ rb_piece  p;
+  __shared__ sm_shared S;
+  unsigned const       lane = threadIdx.x & 31u;
+  uint32_t const       P    = rc->mid;
+  uint32_t             dec  = 0;
+  for (uint32_t pi = blockIdx.x; pi < P; pi += gridDim.x) {
+    uint32_t const root = pieces[cap - 1 - pi], k = count[root], b = start[root];
+    if (threadIdx.x == 0) p.edges = 0;
+    if (threadIdx.x < 6) S.cnt[threadIdx.x >> 1][threadIdx.x & 1] = 0;
+    bool heavy_row = false;
+    for (uint32_t i = threadIdx.x; i < k; i += RB_T) {
       uint32_t const v = members[b + i];
       p.vid[i]         = v;
+      p.out_at[i] = p.in_at[i] = 0;
       heavy_row |= fh[v + 1] - fh[v] > HEAVY_ROW;
     }
-    if (__any_sync(0xFFFFFFFFu, heavy_row)) {
-      // a member's row is too long for one lane: left to the later rounds
-      if (lane == 0) atomicAdd(big, 1u);
-      __syncwarp();
+    // a member's row is too long for a few lanes: left to the later rounds
+    bool left = __syncthreads_or(heavy_row);
+    // internal edges, four lanes per vertex (undecided neighbours lie in this
+    // piece, and nobody else decides them)
+    for (uint32_t i = threadIdx.x >> 2; i < k && !left; i += RB_T / 4) {
+      uint32_t const v = p.vid[i];
+      uint64_t const end = fh[v + 1];
+      for (uint64_t e = fh[v] + (lane & 3u); e < end; e += 4) {
+        uint32_t const w = fc[e];
+        if (!und_has(und, w)) continue;
+        uint32_t const at = atomicAdd(&p.edges, 1u);
+        if (at >= RS_MAXE) break;
+        uint32_t const j = place[w];
+        p.edge[at]       = i << 16 | j;
+        atomicAdd(p.out_at + i, 1u);
+        atomicAdd(p.in_at + j, 1u);
+      }
+    }
+    __syncthreads();
+    uint32_t const m = p.edges;
+    if (left || m > RS_MAXE) {
+      if (threadIdx.x == 0) atomicAdd(big, 1u);
+      __syncthreads();
       continue;
     }
-    __syncwarp();
-    // internal out-degrees; lane l owns local vertices [l*per, l*per + per)
-    uint32_t const per = (k + 31) / 32;
-    uint32_t       cnt = 0;
-    for (uint32_t i = lane * per; i < k && i < lane * per + per; ++i) {
-      uint32_t const v = p.vid[i];
-      uint32_t       c = 0;
-      for (uint64_t e = fh[v], end = fh[v + 1]; e < end; ++e) {
-        uint32_t const w = fc[e];
-        c += und_has(und, w) ? 1u : 0u; // undecided neighbours lie in this piece
-      }
-      p.comp[i] = static_cast<uint16_t>(c < RS_MAXE ? c : RS_MAXE); // clamped; the total decides
-      cnt += c;
-    }
-    uint32_t incl = cnt;
+    // offsets: warp 0 the out-rows', warp 1 the in-rows'
+    if (threadIdx.x < 64) {
+      uint32_t* const at  = threadIdx.x < 32 ? p.out_at : p.in_at;
+      uint16_t* const hd  = threadIdx.x < 32 ? p.fh : p.bh;
+      uint32_t        run = 0;
+      for (uint32_t i0 = 0; i0 < k; i0 += 32) {
+        uint32_t const i = i0 + lane, c = i < k ? at[i] : 0u;
+        uint32_t       incl = c;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      uint32_t const y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-      if (lane >= static_cast<unsigned>(d)) incl += y;
-    }
-    uint32_t const total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    if (total > RS_MAXE) {
-      if (lane == 0) atomicAdd(big, 1u);
-      __syncwarp();
-      continue;
-    }
-    // offsets, then the local adjacency
-    uint32_t run = incl - cnt;
-    for (uint32_t i = lane * per; i < k && i < lane * per + per; ++i) {
-      p.off[i] = static_cast<uint16_t>(run);
-      run += p.comp[i];
-    }
-    if (lane == 0) p.off[k] = static_cast<uint16_t>(total);
-    __syncwarp();
-    for (uint32_t i = lane * per; i < k && i < lane * per + per; ++i) {
-      uint32_t const v = p.vid[i];
-      uint32_t       o = p.off[i];
-      for (uint64_t e = fh[v], end = fh[v + 1]; e < end; ++e) {
-        uint32_t const w = fc[e];
-        if (und_has(und, w)) p.adj[o++] = static_cast<uint16_t>(place[w]);
+        for (int d = 1; d < 32; d <<= 1) {
+          uint32_t const y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+          if (lane >= static_cast<unsigned>(d)) incl += y;
+        }
+        if (i < k) at[i] = run + incl - c, hd[i] = static_cast<uint16_t>(run + incl - c);
+        run += __shfl_sync(0xFFFFFFFFu, incl, 31);
       }
+      if (lane == 0) hd[k] = static_cast<uint16_t>(run);
     }
-    __syncwarp();
-    if (lane == 0) rs_tarjan(p, k);
-    __syncwarp();
-    // an SCC's smallest vertex, gathered at its representative in the piece's
-    // spent index / low arrays (16 bits each: a 32-bit slot per vertex)
-    auto* const least = reinterpret_cast<uint32_t*>(p.index);
-    for (uint32_t i = lane; i < k; i += 32) least[i] = UNDECIDED;
-    __syncwarp();
-    for (uint32_t i = lane; i < k; i += 32) atomicMin(least + p.comp[i], p.vid[i]);
-    __syncwarp();
-    // ids and und; each vertex's word cleared by an atomic (pieces share words)
-    for (uint32_t i = lane; i < k; i += 32) {
-      uint32_t const v = p.vid[i];
-      scc_id[v]        = least[p.comp[i]];
-      atomicAnd(und + (v >> 5), ~(1u << (v & 31)));
+    for (uint32_t w = threadIdx.x; w < (k + 31) / 32; w += RB_T) p.und[w] = k - w * 32 >= 32 ? 0xFFFFFFFFu : (1u << (k & 31)) - 1u;
+    for (uint32_t i = threadIdx.x; i < k; i += RB_T) scc_id[p.vid[i]] = p.vid[i];
+    __syncthreads();
+    for (uint32_t x = threadIdx.x; x < m; x += RB_T) {
+      uint32_t const i = p.edge[x] >> 16, j = p.edge[x] & 0xFFFFu;
+      p.fc[atomicAdd(p.out_at + i, 1u)] = static_cast<uint16_t>(j);
+      p.bc[atomicAdd(p.in_at + j, 1u)]  = static_cast<uint16_t>(i);
     }
-    dec += lane == 0 ? k : 0;
-    __syncwarp();
+    __syncthreads();
+    sm_graph G{ k, (k + 31) / 32, p.lab, p.und, p.open, p.vis, p.inq, p.q0, p.q1, p.fh, p.bh, p.fc, p.bc, &S, 0 };
+    auto const name  = [&](uint32_t v) { return p.vid[v]; };
+    uint32_t   rem   = k - sm_trim<RB_T>(G), edges = 0;
+    for (uint32_t round = 0; rem; ++round) { // a round decides at least one component
+      uint32_t d = sm_label_round<RB_T>(G, round, scc_id, name, edges);
+      if (d < rem) d += sm_trim<RB_T>(G);
+      rem -= d;
+    }
+    // each vertex's word cleared by an atomic (pieces share words)
+    for (uint32_t i = threadIdx.x; i < k; i += RB_T) atomicAnd(und + (p.vid[i] >> 5), ~(1u << (p.vid[i] & 31)));
+    dec += threadIdx.x == 0 ? k : 0u;
+    __syncthreads();
   }
-  if (lane == 0 && dec) atomicAdd(decided, dec);
+  if (threadIdx.x == 0 && dec) atomicAdd(decided, dec);
 }
 
 } // namespace
@@ -447,10 +462,8 @@ residual(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, ui
   k_res_small<<<std::min<unsigned>(148 * 8, rs_grid(undecided * 16)), RS_THREADS, 0, s>>>(rc, pieces, count, start, place, parent, members, g.fh, g.fc, und, scc_id, ws.ctr + CTR_DECIDED,
                                                                                        ws.ctr + CTR_AUX);
   if (undecided > 32) {
-    size_t const smem = sizeof(rs_piece) * RS_WARPS;
-    KSPN_CUDA(cudaFuncSetAttribute(k_res_tarjan, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    k_res_tarjan<<<static_cast<unsigned>(std::min<uint64_t>(148 * 4, undecided / (33 * RS_WARPS) + 1)), RS_WARPS * 32, smem, s>>>(rc, pieces, static_cast<uint32_t>(each), count, start, place, members, g.fh,
-                                                                                                                      g.fc, und, scc_id, ws.ctr + CTR_DECIDED, ws.ctr + CTR_AUX);
+    k_res_block<<<static_cast<unsigned>(std::min<uint64_t>(148 * 6, undecided / 33 + 1)), RB_T, 0, s>>>(rc, pieces, static_cast<uint32_t>(each), count, start, place, members, g.fh, g.fc, und, scc_id,
+                                                                                                       ws.ctr + CTR_DECIDED, ws.ctr + CTR_AUX);
     ctx->launches += 1;
   }
   KSPN_CHECK_LAUNCH();
