@@ -322,7 +322,7 @@ struct workspace
   uint32_t* seed_q      = nullptr; // 4: the pivot as a one-vertex frontier
   uint64_t* seed_prefix = nullptr; // 4
   uint32_t* links       = nullptr; // 4096: links between the start vertices of a worklist phase (reach.cu)
-  void*     gbar        = nullptr; // 4 KiB: grid barrier of the persistent FW-BW at 0, worklist counters at 1024 (zeroed at creation)
+  void*     gbar        = nullptr; // 4 KiB: grid barrier of the persistent FW-BW at 0, worklist counters at 1024, saved level control at 2048, the resume launch's barrier at 3072 (zeroed at creation)
   void*     aw          = nullptr; // aw_entries u64: worklist of the asynchronous search tail (zeroed at creation, zero outside a phase)
   size_t    aw_entries  = 0;       // 4 (n + 2) + 2 AW_STALE vertex items (FW and BW at once, duplicate pushes) + 4 m / HEAVY_SLICE + 128 row-slice items
   void*     rstate      = nullptr; // 4 KiB device control blocks (FW-BW at 0, trim at 512, search stamps at 2048)

@@ -112,6 +112,7 @@ struct reach_state
   uint32_t           restricts;    // passes that cut one search's candidates down to the other's set
   uint32_t           pivot_rejected; // the pivot model rejected the launch's pivot: the launch ended after its first level
   uint32_t           handoff;        // the launch ended where its worklist phase starts; a resume launch continues
+  uint32_t           resumed;        // a resume launch has continued it
 };
 
 // phase stamps live after the state: uint32 phase[128], uint64 ns[128]
@@ -734,7 +735,7 @@ __shared__ unsigned long long s_epoch0;
 // drop-th barrier of the launch without arriving (the test hook of
 // kspn_options.drop_barrier), so the others' waits run out.
 __device__ __forceinline__ bool
-grid_sync(grid_barrier* b, unsigned long long& epoch, unsigned limit, unsigned drop)
+grid_sync(grid_barrier* b, uint32_t* err, unsigned long long& epoch, unsigned limit, unsigned drop)
 {
   __shared__ uint32_t s_ok;
   __syncthreads();
@@ -746,8 +747,8 @@ grid_sync(grid_barrier* b, unsigned long long& epoch, unsigned limit, unsigned d
       asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&b->root), "l"(1ull) : "memory");
       unsigned long long const target = epoch * gridDim.x;
       for (unsigned spins = 0; ld_acquire64(&b->root) < target; ++spins) {
-        if (spins > limit || ((spins & 63u) == 63u && ld_acquire(&b->err))) {
-          atomicExch(&b->err, 1u);
+        if (spins > limit || ((spins & 63u) == 63u && ld_acquire(err))) {
+          atomicExch(err, 1u);
           ok = 0;
           break;
         }
@@ -816,6 +817,7 @@ struct fwbw_args
   uint32_t*          cutmap;    // FW search's cut rows; the BW search's follow at cutmap + cut_words
   uint32_t           cut_words;
   grid_barrier*      bar;
+  uint32_t*          err; // 1: a wait reached the wait limit (the first launch's barrier's word, for the resume launch too)
   reach_state*       st;
   uint32_t*          stamp_phase;
   uint64_t*          stamp_ns;
@@ -838,7 +840,7 @@ struct fwbw_args
 __device__ __forceinline__ bool
 gsync(fwbw_args const& a, unsigned long long& epoch)
 {
-  return grid_sync(a.bar, epoch, a.wait_limit, a.drop_barrier);
+  return grid_sync(a.bar, a.err, epoch, a.wait_limit, a.drop_barrier);
 }
 
 // Block-shared scratch of the persistent kernel.
@@ -1487,8 +1489,8 @@ run_async(fwbw_args const& a, uint32_t const* fq0, uint32_t qn0, aw_dir const d0
         unsigned long long const dn = ld_acquire64(done);
         unsigned long long const t  = ld_acquire64(tail);
         stop                        = dn == t ? 1u : 0u;
-        if (!stop && (spins > a.wait_limit || ((spins & 63u) == 63u && ld_acquire(&a.bar->err)))) {
-          atomicExch(&a.bar->err, 1u);
+        if (!stop && (spins > a.wait_limit || ((spins & 63u) == 63u && ld_acquire(a.err)))) {
+          atomicExch(a.err, 1u);
           stop = 2;
         }
       }
@@ -2438,8 +2440,8 @@ run_trim_async(fwbw_args const& a, uint32_t const* fq, uint32_t qn, unsigned lon
           unsigned long long const dn = ld_acquire64(done);
           unsigned long long const t  = ld_acquire64(tail);
           stop                        = dn == t ? 1u : 0u;
-          if (!stop && (++spins > a.wait_limit || ((spins & 63u) == 63u && ld_acquire(&a.bar->err)))) {
-            atomicExch(&a.bar->err, 1u);
+          if (!stop && (++spins > a.wait_limit || ((spins & 63u) == 63u && ld_acquire(a.err)))) {
+            atomicExch(a.err, 1u);
             stop = 2;
           }
         }
@@ -2563,6 +2565,7 @@ k_fwbw(fwbw_args const __grid_constant__ a)
 {
   __shared__ fwbw_smem sm;
   if (a.gate && __ldcg(a.gate)) return; // the same word for every block
+  if (a.resume && !__ldcg(&a.st->handoff)) return; // queued ahead of need (the same word, too)
   reach_state* const   st    = a.st;
   unsigned long long   epoch = __ldcg(&a.bar->epoch);
   uint32_t const       words = (a.n + 31) / 32;
@@ -2577,7 +2580,7 @@ k_fwbw(fwbw_args const __grid_constant__ a)
   bool const search = p < a.n; // block-uniform
   // a resume launch numbers its barriers on from the launch it continues
   if (threadIdx.x == 0) sm.buf_n = 0, sm.edges_bu = sm.cands_bu = 0, s_epoch0 = a.resume ? epoch - static_cast<joint_save const*>(a.jsave)->barriers : epoch;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && a.resume) st->handoff = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && a.resume) st->resumed = 1;
   if (blockIdx.x == 0 && threadIdx.x == 0 && !a.resume) {
     st->t_ns[0] = globaltimer();
     st->marks   = 0;
@@ -2597,7 +2600,7 @@ k_fwbw(fwbw_args const __grid_constant__ a)
     st->async_phases            = 0;
     st->cut_n[0] = st->cut_n[1] = st->fixups = 0;
     st->hseed_n = st->heavy_err = st->trim_async = st->joint = st->restricts = 0;
-    st->pivot_rejected = st->handoff = 0;
+    st->pivot_rejected = st->handoff = st->resumed = 0;
     for (int i = 0; i < 6; ++i) st->hq_n[i] = 0;
     if (search) a.seed.q[0] = p, a.seed.prefix[0] = 0;
   }
@@ -2947,6 +2950,30 @@ release_graphs(kspn_context* ctx)
 
 namespace {
 
+// The launch that continues one that handed off its worklist phase (same
+// arguments, 80 registers per thread, a grid barrier of its own); without a
+// handoff it ends at once.  Below a mean degree of RESUME_DEGREE most searches
+// hand off (random graphs end in long thin levels, road-like ones consist of
+// them), so it is queued right behind the first launch, without the host
+// round trip between: G(n, m) n 20,000, degree 4: 194 -> 174 us, n 1 M,
+// degree 5: 350 -> 324, random geometric graph n 50,000: 774 -> 748.  Where it
+// is not needed it costs 4 to 5 us (R-MAT scale 16, degree 4: 137 -> 142; at a
+// limit of 8 also G(n, m) n 65,536, degree 8: 150 -> 154).
+constexpr uint64_t RESUME_DEGREE = 6;
+
+void
+launch_resume(kspn_context* ctx)
+{
+  fwbw_args a;
+  std::memcpy(&a, ctx->fwbw_last, sizeof(a));
+  a.resume     = 1;
+  a.bar        = reinterpret_cast<grid_barrier*>(static_cast<char*>(ctx->ws.gbar) + 3072); // its own: the grids differ
+  void* args[] = { &a };
+  KSPN_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(&k_fwbw<3, false>), dim3(resume_grid(ctx)), dim3(R_THREADS), args, 0, ctx->stream));
+  ctx->launches += 1;
+  if (ctx->fwbw_after) KSPN_CUDA(cudaEventRecord(ctx->fwbw_after, ctx->stream));
+}
+
 // Launches k_fwbw (pivot, or PIVOT_FROM_DEVICE; trim tail on or off) and
 // queues the copies of its results into the pinned state mirror; the
 // caller synchronises, then calls check_persistent.
@@ -3001,6 +3028,7 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
   a.cutmap      = ws.cutmap;
   a.cut_words   = static_cast<uint32_t>((static_cast<size_t>(ws.n_cap) + 63) / 64 * 2 + 2);
   a.bar         = gbar;
+  a.err         = &gbar->err;
   a.st          = rs;
   a.stamp_phase = reinterpret_cast<uint32_t*>(static_cast<char*>(ws.rstate) + 2048);
   a.stamp_ns    = reinterpret_cast<uint64_t*>(static_cast<char*>(ws.rstate) + 2048 + 4 * MARKS);
@@ -3021,7 +3049,7 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
   a.label_n      = (static_cast<uint64_t>(g.n) + 15) & ~15ull;
   a.links        = ws.links;
   static_assert(sizeof(fwbw_args) <= sizeof(ctx->fwbw_last), "launch arguments must fit their copy in the context");
-  static_assert(sizeof(joint_save) <= 2048, "saved level control must fit its workspace slot");
+  static_assert(sizeof(joint_save) <= 1024, "saved level control must fit its workspace slot");
   std::memcpy(ctx->fwbw_last, &a, sizeof(a));
   ctx->fwbw_after = after_kernel;
   void* args[]    = { &a };
@@ -3030,6 +3058,7 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
   KSPN_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(fwbw_grid(ctx, g)), dim3(R_THREADS), args, 0, ctx->stream));
   ctx->launches += 1;
   if (after_kernel) KSPN_CUDA(cudaEventRecord(after_kernel, ctx->stream));
+  if (trim && g.m < RESUME_DEGREE * g.n) launch_resume(ctx);
   // results, and the barrier's error word (read after the launch ended: a
   // block that gave up may set it after block 0 finished)
   auto* const hb = reinterpret_cast<uint32_t*>(static_cast<char*>(ctx->h_state) + 1024);
@@ -3038,25 +3067,17 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
 }
 
 // After the stream was synchronised: a launch that handed off its worklist
-// phase is continued by the resume launch (same arguments, 80 registers
-// per thread; one more host round trip, only on graphs that reach that
-// phase); then barrier failures and level caps.  Returns whether a resume
-// launch ran.
+// phase and has no resume launch behind it yet is continued by one (one more
+// host round trip); then barrier failures and level caps.  Returns whether
+// the host launched one.
 bool
 check_persistent(kspn_context* ctx)
 {
   auto* const hs = reinterpret_cast<reach_state*>(ctx->h_state);
   auto* const hb      = reinterpret_cast<uint32_t*>(static_cast<char*>(ctx->h_state) + 1024);
-  bool const  resumed = hs->handoff && !*hb && !hs->bar_err;
+  bool const  resumed = hs->handoff && !hs->resumed && !*hb && !hs->bar_err;
   if (resumed) {
-    fwbw_args a;
-    std::memcpy(&a, ctx->fwbw_last, sizeof(a));
-    a.resume     = 1;
-    void* args[] = { &a };
-    barrier_for_grid(ctx, resume_grid(ctx));
-    KSPN_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const*>(&k_fwbw<3, false>), dim3(resume_grid(ctx)), dim3(R_THREADS), args, 0, ctx->stream));
-    ctx->launches += 1;
-    if (ctx->fwbw_after) KSPN_CUDA(cudaEventRecord(ctx->fwbw_after, ctx->stream));
+    launch_resume(ctx);
     KSPN_CUDA(cudaMemcpyAsync(hs, ctx->ws.rstate, sizeof(reach_state), cudaMemcpyDeviceToHost, ctx->stream));
     KSPN_CUDA(cudaMemcpyAsync(hb, &static_cast<grid_barrier*>(ctx->ws.gbar)->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
