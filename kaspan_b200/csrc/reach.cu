@@ -430,20 +430,23 @@ bu_sweep_chunk(uint32_t c,
   __syncwarp();
 }
 
-// Bottom-up sweep of the cnt <= BU_GROUP consecutive chunks [c0, c0 + cnt)
-// by one warp (cnt = 1 on dense levels): lane i loads word i of every chunk
+// Bottom-up sweep of cnt <= BU_GROUP consecutive chunks, words [w0, lim), by
+// one warp (cnt = 1 on dense levels): lane i loads word i of every chunk
 // (independent loads); the chunks are then taken in segments of at most
 // 32 x 32 candidates (the pack buffer), each packed once and walked in
 // batches of 32 x BU_ILP as bu_rows does, after which lane i writes back
-// word i of each chunk of the segment.  A chunk is cw words (32, fewer on a
-// graph of too few words to give every warp of the grid one, then cnt = 1).
+// word i of each chunk of the segment.  A chunk is 32 words (fewer on a
+// graph of too few words to give every warp of the grid one, then cnt = 1;
+// only lim knows, so that the dense sweeps keep the constant: with the chunk
+// size as a variable the first one of R-MAT scale 26, 550 us, took about 4
+// more).
 // On a sparse level one segment holds
 // the whole group, so its few candidates share one dependent head ->
 // neighbour -> probe chain instead of one chain per chunk.
 __device__ __forceinline__ void
-bu_sweep_group(uint32_t c0,
+bu_sweep_group(uint32_t w0,
                uint32_t cnt,
-               uint32_t cw,
+               uint32_t lim,
                uint32_t n,
                uint64_t const* __restrict__ head,
                uint32_t const* __restrict__ adj,
@@ -462,8 +465,8 @@ bu_sweep_group(uint32_t c0,
   // segment is packed (no register array across the scans)
 #pragma unroll
   for (int g = 0; g < BU_GROUP; ++g) {
-    uint32_t const w = (c0 + g) * cw + lane;
-    uint32_t       x = static_cast<uint32_t>(g) < cnt && lane < cw && w < words ? __ldcg(avail + w) : 0u;
+    uint32_t const w = w0 + g * 32 + lane;
+    uint32_t       x = w < lim ? __ldcg(avail + w) : 0u;
     if (w == words - 1 && (n & 31)) x &= (1u << (n & 31)) - 1u;
     sm.found[g * 32 + lane] = x;
   }
@@ -497,7 +500,7 @@ bu_sweep_group(uint32_t c0,
     }
     __syncwarp();
     ncand += lane == 0 ? total : 0;
-    uint32_t const vbase = (c0 + s0) * cw * 32;
+    uint32_t const vbase = (w0 + s0 * 32) * 32;
     for (uint32_t r = 0; r < total; r += 32 * BU_ILP) {
       uint32_t v[BU_ILP];
       bool     live[BU_ILP], found[BU_ILP];
@@ -510,13 +513,13 @@ bu_sweep_group(uint32_t c0,
       bu_rows(v, live, found, head, adj, mark, cut, nedge);
 #pragma unroll
       for (int k = 0; k < BU_ILP; ++k)
-        if (found[k]) atomicOr(&sm.found[(v[k] >> 5) - c0 * cw], 1u << (v[k] & 31));
+        if (found[k]) atomicOr(&sm.found[(v[k] >> 5) - w0], 1u << (v[k] & 31));
     }
     __syncwarp();
     for (uint32_t g = s0; g < s1; ++g) {
-      uint32_t const w   = (c0 + g) * cw + lane;
+      uint32_t const w   = w0 + g * 32 + lane;
       uint32_t const fnd = sm.found[g * 32 + lane];
-      if (lane < cw && w < words) {
+      if (w < lim) {
         if (fnd) {
           atomicAnd(avail + w, ~fnd);
           atomicOr(mark + w, fnd);
@@ -1993,9 +1996,9 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
         int const      d  = cc < c0 ? 0 : 1;
         jdir const     D  = joint_dir(a, d);
         uint32_t const gs = d ? g1 : g0;
-        uint32_t const ch = (d ? cc - c0 : cc) * gs;
+        uint32_t const ch = (d ? cc - c0 : cc) * gs, cnt = chunks - ch < gs ? chunks - ch : gs;
         uint32_t       f  = 0;
-        bu_sweep_group(ch, chunks - ch < gs ? chunks - ch : gs, cw, a.n, D.bu_head, D.bu_adj, D.avail, D.mark, D.fresh, s_bu_cut[d], sm.warp[wid], f, ne, ncd);
+        bu_sweep_group(ch * cw, cnt, min(words, (ch + cnt) * cw), a.n, D.bu_head, D.bu_adj, D.avail, D.mark, D.fresh, s_bu_cut[d], sm.warp[wid], f, ne, ncd);
         if (d) nf1 += f;
         else nf0 += f;
       }
