@@ -279,8 +279,8 @@ int kspn_trim_1_fixpoint(kspn_context* ctx, uint32_t n, uint64_t m,
 /* Residual device finish (the residual step of variant/scc_trim_ex_residual.hpp:110-127:
  * allgather_fw_sub_graph + tarjan): the sub-graph induced by the undecided
  * vertices is split into weakly connected pieces, and every piece of at most
- * 512 vertices and 2048 internal edges is decomposed by Tarjan in one warp's
- * shared memory; its SCCs get their smallest member as id and leave
+ * 512 vertices and 2048 internal edges is decomposed in shared memory (a warp's
+ * closure or a block's label rounds); its SCCs get their smallest member as id and leave
  * `undecided`.  *decided = vertices decided, *pieces_left = pieces too large
  * (left undecided); both nullable. */
 int kspn_residual(kspn_context* ctx, uint32_t n, uint64_t m,

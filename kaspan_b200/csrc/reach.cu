@@ -538,7 +538,7 @@ bu_sweep_group(uint32_t w0,
 // walks its chunk's candidates 32 x BU_ILP at a time, each batch one chain
 // of dependent loads: on G(n, m) of 2^16 vertices (64 chunks of 32 words, the
 // other warps idle) the first sweep took 98 us and a whole call 272 us, with
-// small chunks 191 us; on 1000 vertices (one chunk) 243 and 171 us.
+// small chunks 191 us (with grids of four blocks per SM).
 __device__ __forceinline__ uint32_t
 bu_chunk_words(uint32_t words)
 {
@@ -2559,9 +2559,10 @@ write_ids(fwbw_args const& a, uint32_t words, bool search, uint32_t scc)
 // keep their loads in flight without spills: with several start vertices
 // the phase has work for every warp (RGG 2^24, whole call: 2 blocks 6.44 ms,
 // 3: 5.73, 4: 5.37 but slower on shorter phases).
-// THIN: with the thin opening.  A launch of its own for the pivot model, which
-// scores the pivot during a grid-wide first level: the opening's call costs
-// the levels' code 40 bytes of spills (R-MAT scale 26: 1,221 -> 1,233 us).
+// THIN: with the thin opening, whose call costs the levels' code 40 bytes of
+// spills.  Without it for the pivot model, which scores the pivot during a
+// grid-wide first level, and for large dense graphs (R-MAT scale 26: 968
+// instead of 978 us).
 template<int MINB, bool THIN>
 __global__ void __launch_bounds__(R_THREADS, MINB)
 k_fwbw(fwbw_args const __grid_constant__ a)
@@ -2962,6 +2963,7 @@ namespace {
 // degree 5: 350 -> 324, random geometric graph n 50,000: 774 -> 748.  Where it
 // is not needed it costs 4 to 5 us (R-MAT scale 16, degree 4: 137 -> 142; at a
 // limit of 8 also G(n, m) n 65,536, degree 8: 150 -> 154).
+constexpr uint64_t THIN_MAX = 1ull << 29;
 constexpr uint64_t RESUME_DEGREE = 6;
 
 void
@@ -3057,7 +3059,10 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
   ctx->fwbw_after = after_kernel;
   void* args[]    = { &a };
   barrier_for_grid(ctx, fwbw_grid(ctx, g));
-  auto* const kernel = a.model ? reinterpret_cast<void const*>(&k_fwbw<4, false>) : reinterpret_cast<void const*>(&k_fwbw<4, true>);
+  // the opening saves at most three levels (27 us) where the mean degree is 8
+  // and more; on such a graph of THIN_MAX vertices and edges its spills cost as much
+  bool const  thin   = !a.model && (g.m < 8ull * g.n || g.n + g.m < THIN_MAX);
+  auto* const kernel = thin ? reinterpret_cast<void const*>(&k_fwbw<4, true>) : reinterpret_cast<void const*>(&k_fwbw<4, false>);
   KSPN_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(fwbw_grid(ctx, g)), dim3(R_THREADS), args, 0, ctx->stream));
   ctx->launches += 1;
   if (after_kernel) KSPN_CUDA(cudaEventRecord(after_kernel, ctx->stream));
