@@ -94,7 +94,9 @@ typedef struct kspn_options
                                Needs a model and n <= 2^31; same partition either way */
 } kspn_options;
 
-/* Per-call statistics (all fields written by a successful call). */
+/* Per-call statistics (all fields written by a successful call).  A graph that
+ * one block decomposes (kernel_launches 1) has its whole time under FWBW, what
+ * the trim fixpoint leaves under RESIDUAL, and no resident launch. */
 #define KSPN_PHASES 8
 #define KSPN_PHASE_TRIM_FIRST 0
 #define KSPN_PHASE_TRIM 1
