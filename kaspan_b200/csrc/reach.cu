@@ -1116,7 +1116,7 @@ struct aw_sink
 // neither search has reached (seed_start) -- and every vertex keeps the label
 // of the start vertex it was reached from, per direction.  Afterwards C = FW
 // & BW is a union of whole SCCs that contains the pivot's (a vertex on a path
-// between two members is in both sets).  A vertex with FW label i and BW
+// between two members is in both sets; so no row may wait on a cut list).  A vertex with FW label i and BW
 // label j shows that start vertex i reaches j; when the links found that way
 // (seed_links) put every start vertex into one strongly connected set with
 // the pivot, C is the pivot's SCC.  Otherwise the sets restart inside C
@@ -1883,8 +1883,12 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
         // several start vertices where the searches grow slowly and most of the
         // graph is undecided (near the giant-component threshold of a random
         // graph, mean degree below 1.7, less than 2/3 are and most candidates
-        // lie outside the SCC: a restart for nothing); block-uniform
-        bool const seeded = two && a.seeds && !s_j.seeded && static_cast<uint64_t>(n_und) * 3 >= static_cast<uint64_t>(a.n) * 2 && joint_slow(qmask);
+        // lie outside the SCC: a restart for nothing), and no row is on a cut
+        // list: its vertex, and what only it leads to, may belong to the SCC
+        // and be in neither set yet, and a restart would keep them out of C
+        // for good; block-uniform (no sweep runs since the last barrier)
+        bool const seeded = two && a.seeds && !s_j.seeded && static_cast<uint64_t>(n_und) * 3 >= static_cast<uint64_t>(a.n) * 2 && joint_slow(qmask) && __ldcg(&st->cut_n[0]) == 0 &&
+                            __ldcg(&st->cut_n[1]) == 0;
         int const r = run_async(a, f0.q, static_cast<uint32_t>(s_j.c[d0] & qmask), w0, f1.q, static_cast<uint32_t>(s_j.c[1] & qmask), two ? &w1 : nullptr, epoch, ea, sm, seeded);
         if (r != SEARCH_DONE) return r;
         stamp(a, 13);
