@@ -154,7 +154,6 @@ read_counters(kspn_context* ctx)
 {
   KSPN_CUDA(cudaMemcpyAsync(ctx->h_ctr, ctx->ws.ctr, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
   KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
-  look_back_check(ctx);
 }
 
 void
@@ -236,7 +235,6 @@ run_small(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options con
   scc_small_async(ctx, g, scc_id, res);
   if (st) KSPN_CUDA(cudaEventRecord(ctx->ev[1], ctx->stream));
   KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
-  look_back_check(ctx);
   if (res->bad) {
     if (opt.validate) validate_check(res->bad);
     return false;
@@ -426,7 +424,6 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
       fw_bw_trim_async(ctx, g, und, scc_id, opt, st, st ? ctx->ev[4] : nullptr);
       KSPN_CUDA(cudaMemcpyAsync(ctx->h_ctr, ws.ctr, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
       finished();
-      look_back_check(ctx);
       if (opt.validate) validate_check(ctx->h_ctr[CTR_ERR]);
       resident_result r = fw_bw_trim_result(ctx, g, opt, st);
       if (r.resumed) {
@@ -812,7 +809,6 @@ kspn_context_create_on_stream(int device, void* stream, kspn_context** out)
     ctx->h_ctr   = static_cast<uint32_t*>(h);
     ctx->h_ctr64 = reinterpret_cast<uint64_t*>(ctx->h_ctr + 32);
     KSPN_CUDA(cudaMallocHost(&ctx->h_state, 4096));
-    std::memset(ctx->h_state, 0, 4096);
     for (auto& e : ctx->ev) KSPN_CUDA(cudaEventCreate(&e));
     for (auto& e : ctx->pe) KSPN_CUDA(cudaEventCreate(&e));
   });
@@ -859,10 +855,7 @@ int
 kspn_context_synchronize(kspn_context* ctx)
 {
   if (!ctx) return KSPN_ERR_INVALID_ARGUMENT;
-  return guard(ctx, [&] {
-    KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
-    look_back_check(ctx);
-  });
+  return guard(ctx, [&] { KSPN_CUDA(cudaStreamSynchronize(ctx->stream)); });
 }
 
 uint64_t
@@ -1379,7 +1372,6 @@ kspn_upload_transpose(kspn_context* ctx, uint32_t n, uint64_t m, const uint64_t*
     bind_device(ctx);
     upload_transpose(ctx, n, m, fw_head, fw_csr, d_fw_head, d_fw_csr, d_bw_head, d_bw_csr, chunk_edges);
     KSPN_CUDA(cudaStreamSynchronize(ctx->stream));
-    look_back_check(ctx);
   });
 }
 

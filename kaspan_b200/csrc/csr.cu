@@ -609,7 +609,6 @@ build_csr(kspn_context* ctx, uint32_t n, uint64_t m_raw, uint32_t* src, uint32_t
   uint32_t m = 0;
   KSPN_CUDA(cudaMemcpyAsync(&m, cnt + ET_CHUNKS, sizeof(m), cudaMemcpyDeviceToHost, s));
   KSPN_CUDA(cudaStreamSynchronize(s));
-  look_back_check(ctx);
   return m;
 }
 

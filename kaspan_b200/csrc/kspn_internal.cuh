@@ -411,7 +411,7 @@ struct kspn_context
   // kernel-class timing (kspn_options.profile): two event pairs in flight
   kspn_stats*        prof       = nullptr;
   cudaEvent_t        pe[4]      = {};
-  void*              h_state    = nullptr; // pinned 4 KiB: mirror of ws.rstate, trim state at 512, small_result at SMALL_RESULT_AT, look-back fault word last
+  void*              h_state    = nullptr; // pinned 4 KiB: mirror of ws.rstate, trim state at 512, small_result at SMALL_RESULT_AT
   unsigned           search_grid = 0;      // most blocks of the persistent FW-BW launch that are resident at once
   unsigned           search_sms  = 0;
   unsigned           resume_grid = 0;      // blocks of its resume launch (the worklist phase)

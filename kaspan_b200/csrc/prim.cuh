@@ -167,18 +167,6 @@ st_relaxed64(unsigned long long* p, unsigned long long v)
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Error word of kernels with a decoupled look-back (a tile waits for earlier
-// tiles' counts, with a bound): the last word of the context's pinned state
-// mirror, which kernels reach over the unified address space.
-constexpr size_t LOOK_BACK_ERR_AT = 4092;
-inline uint32_t*
-look_back_err(kspn_context* ctx)
-{
-  return reinterpret_cast<uint32_t*>(static_cast<char*>(ctx->h_state) + LOOK_BACK_ERR_AT);
-}
-// After the stream was synchronised: throws if a look-back gave up.
-void look_back_check(kspn_context* ctx);
-
 // radix.cu: stable LSD radix sort of (key, value) u32 pairs on key bits
 // [begin_bit, end_bit).  The result ends in keys/vals; keys_alt/vals_alt
 // are scratch of the same size.  hist needs radix_hist_entries(count).

@@ -10,7 +10,10 @@
 //      counters of its own in shared memory (no block barrier per step);
 //   2. the tile's digit counts are published, and the threads of the first
 //      256 walk back over earlier tiles' words, one digit each, adding counts
-//      until they meet an inclusive prefix; then they publish theirs;
+//      until they meet an inclusive prefix; then they publish theirs.  A
+//      thread that has polled in vain RX_POLLS times takes the missing counts
+//      from the earlier tiles' keys, which stay as they are during a pass: a
+//      wait ends in any case, and with the right sum;
 //   3. keys, then values, are staged in shared memory in digit order and
 //      written as runs of consecutive addresses.
 // Bound: 16 B per pair and pass over HBM; what it spends is issue slots (8
@@ -46,7 +49,7 @@ constexpr size_t             RX_HEAD   = RX_PASSES * RX_BINS + 64;
 constexpr unsigned long long RX_SUM    = 1ull << 32; // the tile's own count
 constexpr unsigned long long RX_PREFIX = 2ull << 32; // the count of all tiles up to it
 constexpr uint32_t           RX_LOOK   = 4;          // look-back words a thread loads at once
-constexpr unsigned           RX_SPINS  = 1u << 22;   // polls before a look-back gives up
+constexpr uint32_t           RX_POLLS  = 1u << 20;   // polls in vain (some tenths of a second) before a look-back counts keys instead
 
 struct rx_digits
 {
@@ -162,7 +165,7 @@ struct rx_args
   uint32_t const*     hist;   // this pass's digit counts
   uint32_t*           ticket; // this pass's
   unsigned long long* look;   // RX_BINS words per tile
-  uint32_t*           err;    // host-mapped; 1: a look-back gave up
+  uint32_t            polls;  // RX_POLLS
 };
 
 // One tile of n pairs (FULL: all RX_TILE of them, no bounds checks).
@@ -230,10 +233,9 @@ rx_tile(rx_args const& a, rx_smem& sm, uint32_t tile, uint32_t n)
 #pragma unroll
   for (int r = 0; r < RX_ITEMS; ++r) val[r] = FULL || first + r * 32 < n ? vin[r * 32] : 0u;
   if (tile && t < RX_BINS) {
-    uint32_t sum   = 0;
-    unsigned spins = 0;
-    bool     done  = false;
-    for (uint32_t j = tile; j > 0 && !done;) {
+    uint32_t sum = 0, polls = 0, j = tile;
+    bool     done = false;
+    while (j > 0 && !done) {
       // RX_LOOK earlier tiles' words in flight at once
       unsigned long long x[RX_LOOK];
 #pragma unroll
@@ -247,10 +249,15 @@ rx_tile(rx_args const& a, rx_smem& sm, uint32_t tile, uint32_t n)
           ++taken;
         }
       j -= taken;
-      if (taken == 0 && ++spins > RX_SPINS) {
-        *reinterpret_cast<uint32_t volatile*>(a.err) = 1u; // a sum too small: every position below stays inside the output
-        done                                         = true;
-      }
+      if (taken == 0 && ++polls > a.polls) break;
+    }
+    if (!done) {
+      // waited for tile j - 1 in vain: its count and all before it from the
+      // keys, and the digits below
+#pragma unroll 4
+      for (uint64_t i = 0, end = static_cast<uint64_t>(j) * RX_TILE; i < end; ++i) sum += ((a.kin[i] >> a.shift) & a.mask) == t;
+#pragma unroll 1
+      for (uint32_t d = 0; d < t; ++d) sum += a.hist[d];
     }
     sm.base[t] = sum - off;
     st_relaxed64(a.look + static_cast<uint64_t>(tile) * RX_BINS + t, tag | RX_PREFIX | static_cast<uint32_t>(sum + c));
@@ -277,7 +284,7 @@ rx_tile(rx_args const& a, rx_smem& sm, uint32_t tile, uint32_t n)
 }
 
 __global__ void __launch_bounds__(RX_THREADS, RX_BLOCKS)
-k_radix_pass(rx_args a)
+k_radix_pass(rx_args const __grid_constant__ a)
 {
   __shared__ rx_smem sm;
   if (threadIdx.x == 0) sm.tile = atomicAdd(a.ticket, 1u);
@@ -305,7 +312,7 @@ void
 rx_pass(kspn_context* ctx, rx_digits const& d, int p, uint32_t const* kin, uint32_t const* vin, uint32_t* kout, uint32_t* vout, uint64_t count, uint32_t* scratch)
 {
   k_radix_pass<<<div_up(count, RX_TILE), RX_THREADS, 0, ctx->stream>>>(rx_args{ kin, vin, kout, vout, count, d.shift[p], d.mask[p], p, scratch + p * RX_BINS, scratch + RX_PASSES * RX_BINS + p,
-                                                                              reinterpret_cast<unsigned long long*>(scratch + RX_HEAD), look_back_err(ctx) });
+                                                                              reinterpret_cast<unsigned long long*>(scratch + RX_HEAD), RX_POLLS });
   KSPN_CHECK_LAUNCH();
   ctx->launches += 1;
 }
@@ -322,15 +329,6 @@ int
 radix_passes(int begin_bit, int end_bit)
 {
   return end_bit > begin_bit ? (end_bit - begin_bit + 7) / 8 : 0;
-}
-
-void
-look_back_check(kspn_context* ctx)
-{
-  uint32_t volatile* const e = look_back_err(ctx);
-  if (!*e) return;
-  *e = 0;
-  throw error{ KSPN_ERR_TIMEOUT, "sort: a look-back wait limit was reached" };
 }
 
 bool
