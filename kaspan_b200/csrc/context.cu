@@ -227,8 +227,8 @@ struct phase_clock
 bool
 run_small(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options const& opt, kspn_stats* st)
 {
-  if (opt.pipeline != KSPN_PIPELINE_FAST || ctx->union_route || (opt.learned_pivot && ctx->pivot_model) || opt.profile || opt.trace || opt.max_levels || opt.max_rounds || opt.wait_limit ||
-      opt.drop_barrier || opt.aw_exact_after || !small_fits(g))
+  if (opt.pipeline != KSPN_PIPELINE_FAST || ctx->union_route || (opt.learned_pivot && ctx->pivot_model) || opt.profile || opt.trace || opt.max_levels || opt.max_rounds || opt.max_label_iters ||
+      opt.wait_limit || opt.drop_barrier || opt.aw_exact_after || !small_fits(g))
     return false;
   auto* const res = reinterpret_cast<small_result*>(static_cast<char*>(ctx->h_state) + SMALL_RESULT_AT);
   if (st) KSPN_CUDA(cudaEventRecord(ctx->ev[0], ctx->stream));
