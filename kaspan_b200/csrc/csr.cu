@@ -15,9 +15,10 @@ namespace kspn {
 namespace {
 
 // src[e] = u for every edge e of row u.  Small rows by their own lane,
-// rows of 64+ entries by the whole warp.
+// rows of 64+ entries by the whole warp.  The offsets may not have been
+// checked yet: nothing past src[m) is written.
 __global__ void
-k_expand_rows(uint32_t n, uint64_t const* __restrict__ head, uint32_t* __restrict__ src)
+k_expand_rows(uint32_t n, uint64_t m, uint64_t const* __restrict__ head, uint32_t* __restrict__ src)
 {
   uint64_t const tid  = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   unsigned const lane = threadIdx.x & 31u;
@@ -25,7 +26,7 @@ k_expand_rows(uint32_t n, uint64_t const* __restrict__ head, uint32_t* __restric
   if (wbase >= n) return;
   uint32_t const u   = static_cast<uint32_t>(tid);
   bool const     ok  = tid < n;
-  uint64_t const beg = ok ? head[u] : 0, end = ok ? head[u + 1] : 0;
+  uint64_t const end = ok ? min(head[u + 1], m) : 0, beg = ok ? min(head[u], end) : 0;
   bool const     big = (end - beg) >= 64;
   if (!big)
     for (uint64_t e = beg; e < end; ++e) src[e] = u;
@@ -476,7 +477,7 @@ transpose(kspn_context* ctx, uint32_t n, uint64_t m, uint64_t const* fh, uint32_
   int const passes = m ? radix_passes(0, bits_for(n)) : 0;
   if (m) {
     uint32_t* const src = passes % 2 ? va : bc;
-    k_expand_rows<<<div_up(n, 256), 256, 0, s>>>(n, fh, src);
+    k_expand_rows<<<div_up(n, 256), 256, 0, s>>>(n, m, fh, src);
     KSPN_CHECK_LAUNCH();
     radix_sort_pairs_to(ctx, fc, src, kb, bc, ka, va, kb, bc, m, bits_for(n), hist);
   }
