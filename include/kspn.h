@@ -151,7 +151,10 @@ typedef struct kspn_stats
    * ended there: 0 launch start, 8 init, 4 expansion level (top-down),
    * 5 sweep level (bottom-up), 7 frontier built from a sweep's bitmap,
    * 10 SCC written back, 11 trim live degrees + seeds, 12 trim push
-   * level, 9 launch end. */
+   * level, 13 worklist phase, 14 fix-up of rows cut short, 15 heavy rows'
+   * live degrees, 16 trim's worklist phase, 17 links between a worklist
+   * phase's start vertices, 18 first levels, run by one block, handed to
+   * the grid, 9 launch end. */
   uint32_t search_marks;
   uint32_t search_phase[128];
   uint64_t search_ns[128];

@@ -1766,6 +1766,7 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
       auto const* const js = static_cast<joint_save const*>(a.jsave);
       if (threadIdx.x == 0 && blockIdx.x) s_j = js->j;
       glvl = __ldcg(&js->glvl);
+      stamp(a, 18);
     }
   }
   int  rc         = SEARCH_DONE;
