@@ -407,8 +407,8 @@ typedef struct kspn_batch_options {
 } kspn_batch_options;
 
 typedef struct kspn_batch_stats {
-    uint32_t graphs_small;  /* decomposed by one warp */
-    uint32_t graphs_large;  /* decomposed by one block */
+    uint32_t graphs_small;  /* decomposed by one warp: at most 32 vertices and 2048 edges */
+    uint32_t graphs_large;  /* all others: by one block, or a cluster of them */
     uint32_t fwbw_rounds;   /* FW-BW rounds over all large graphs */
     uint32_t tarjan_smem;   /* remainders finished in shared memory */
     uint32_t tarjan_serial; /* remainders finished by one thread (round cap) */

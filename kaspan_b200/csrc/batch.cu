@@ -1028,7 +1028,7 @@ bb_trim(uint32_t* err, bb_block& B, uint32_t* q0, bb_degrees const deg, bb_rows 
       break;
     }
     uint32_t* const counter = &B.S->cnt[B.level % 3];
-bb_rows const rows[2] = { fw, bw }; // out-rows lower in-degrees, in-rows out-degrees
+    bb_rows const   rows[2] = { fw, bw }; // out-rows lower in-degrees, in-rows out-degrees
     bb_expand<T>(list, lo, hi, rows, q0, at, counter, [&](uint32_t const (&w)[2 * BB_ILP]) {
       uint32_t left[2 * BB_ILP], found = 0;
 #pragma unroll

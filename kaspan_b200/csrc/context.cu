@@ -466,8 +466,8 @@ run_pipeline(kspn_context* ctx, dgraph const& g, uint32_t* scc_id, kspn_options 
       trimmed     = true;
       und_checked = decided == g.n; // the launch counted und: empty
       if (decided < g.n) fwbw_again();
-      // what is left splits into small pieces on most graphs: Tarjan per
-      // piece in shared memory; larger pieces go on to the rounds below
+      // what is left splits into small pieces on most graphs: each one by a
+      // warp or a block; larger pieces go on to the rounds below
       if (decided < g.n) add(KSPN_PHASE_RESIDUAL, residual(ctx, g, und, scc_id, nullptr, g.n - decided));
     } else {
       uint32_t pivot = trim_1_first(ctx, g, und, scc_id, nullptr, nullptr, false);

@@ -539,8 +539,9 @@ void mlp_forward(kspn_context* ctx, uint32_t count, float const* feat, float con
 void mlp_grad(kspn_context* ctx, uint32_t count, float const* feat, float const* y, float const* params, float* grad, float* loss);
 void mlp_adam(kspn_context* ctx, float* params, float const* grad, float* m, float* v, float lr, int step);
 void learned_pivot(kspn_context* ctx, dgraph const& g, float const* params, bool check = true);
-// residual.cu: Tarjan per weakly connected undecided piece that fits a warp's
-// shared memory; returns vertices decided, *pieces_left = pieces left over
+// residual.cu: every weakly connected undecided piece of at most RS_MAXV
+// vertices and RS_MAXE edges (a warp's closure or a block's label rounds);
+// returns vertices decided, *pieces_left = pieces left over
 uint32_t residual(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t* pieces_left, uint64_t undecided);
 void     count_undecided_async(kspn_context* ctx, uint32_t n, uint32_t const* und); // into ws.ctr[CTR_LEFT]
 

@@ -1125,12 +1125,12 @@ struct aw_sink
 // searches go on among the other vertices of C from a bottom-up sweep until
 // nothing joins.  Both ways FW & BW is exactly the pivot's SCC.
 
-// The first blocks's threads try one candidate each: it starts in both
+// The first block's threads try one candidate each: it starts in both
 // directions if both searches may still reach it.  Its two items follow the
 // frontiers' (from `at`).  Returns the items' end (block 0 only; the other
 // blocks return `at`).  All threads of every block call it.
 __device__ __forceinline__ unsigned long long
-seed_start(fwbw_args const& a, unsigned long long* aw, unsigned long long at, fwbw_smem& sm)
+seed_start(fwbw_args const& a, unsigned long long* aw, unsigned long long at)
 {
   for (int i = blockIdx.x * R_THREADS + threadIdx.x; i < LINK_WORDS - 8; i += gridDim.x * R_THREADS) a.links[i] = 0;
   if (blockIdx.x != 0) return at;
@@ -1158,7 +1158,6 @@ seed_start(fwbw_args const& a, unsigned long long* aw, unsigned long long at, fw
     __stcg(aw + at + 2 * r, item);
     __stcg(aw + at + 2 * r + 1, item | AW_BW);
   }
-  (void)sm;
   return at + 2 * tot;
 }
 
@@ -1310,7 +1309,7 @@ run_async(fwbw_args const& a, uint32_t const* fq0, uint32_t qn0, aw_dir const d0
     __stcg(aw + i, i < qn0 ? AW_TAG | AW_TAKEN | __ldcg(fq0 + i) : AW_TAG | AW_TAKEN | AW_BW | __ldcg(fq1 + (i - qn0)));
   unsigned long long first = qn0 + qb;
   if (seeded) {
-    first = seed_start(a, aw, first, sm);
+    first = seed_start(a, aw, first);
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * R_THREADS + threadIdx.x; i < 2 * a.label_n / 16; i += static_cast<uint64_t>(gridDim.x) * R_THREADS)
       __stcg(reinterpret_cast<uint4*>(a.label) + i, make_uint4(0, 0, 0, 0)); // everything reached so far: the pivot's
   }

@@ -247,8 +247,7 @@ k_res_members(uint32_t const* __restrict__ list, uint32_t const* __restrict__ li
 // still counts as its own piece's).
 __global__ void __launch_bounds__(RS_THREADS)
 k_res_small(rs_counts const* __restrict__ rc, uint32_t const* __restrict__ pieces, uint32_t const* __restrict__ count, uint32_t const* __restrict__ start, uint32_t const* __restrict__ place,
-            uint32_t const* __restrict__ parent, uint32_t const* __restrict__ members, uint64_t const* __restrict__ fh, uint32_t const* __restrict__ fc, uint32_t* und, uint32_t* __restrict__ scc_id,
-            uint32_t* decided, uint32_t* big)
+            uint32_t const* __restrict__ members, uint64_t const* __restrict__ fh, uint32_t const* __restrict__ fc, uint32_t* und, uint32_t* __restrict__ scc_id, uint32_t* decided, uint32_t* big)
 {
   unsigned const lane = threadIdx.x & 31u;
   uint32_t const P    = rc->small;
@@ -303,7 +302,6 @@ k_res_small(rs_counts const* __restrict__ rc, uint32_t const* __restrict__ piece
     }
     dec += lane == 0 ? k : 0u;
   }
-  (void)parent;
   if (lane == 0 && dec) atomicAdd(decided, dec);
 }
 
@@ -416,8 +414,9 @@ k_res_block(rs_counts const* __restrict__ rc, uint32_t const* __restrict__ piece
 } // namespace
 
 // Decides every undecided piece (weakly connected component of the
-// undecided sub-graph) that fits a warp's shared memory; returns the
-// vertices decided.  `undecided` (n when not known) sizes the launches.  *pieces_left (nullable) = pieces left undecided.
+// undecided sub-graph) of at most RS_MAXV vertices and RS_MAXE internal edges;
+// returns the vertices decided.  `undecided` (n when not known) sizes the
+// launches.  *pieces_left (nullable) = pieces left undecided.
 uint32_t
 residual(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, uint32_t* pieces_left, uint64_t undecided)
 {
@@ -459,8 +458,7 @@ residual(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* scc_id, ui
   k_res_flatten<<<grid, RS_THREADS, 0, s>>>(list, &rc->list_n, parent, count, place, ws.ctr + CTR_ERR);
   k_res_ranges<<<grid, RS_THREADS, 0, s>>>(list, parent, count, start, pieces, static_cast<uint32_t>(each), rc, ws.ctr + CTR_AUX);
   k_res_members<<<grid, RS_THREADS, 0, s>>>(list, &rc->list_n, parent, start, place, members);
-  k_res_small<<<std::min<unsigned>(148 * 8, rs_grid(undecided * 16)), RS_THREADS, 0, s>>>(rc, pieces, count, start, place, parent, members, g.fh, g.fc, und, scc_id, ws.ctr + CTR_DECIDED,
-                                                                                       ws.ctr + CTR_AUX);
+  k_res_small<<<std::min<unsigned>(148 * 8, rs_grid(undecided * 16)), RS_THREADS, 0, s>>>(rc, pieces, count, start, place, members, g.fh, g.fc, und, scc_id, ws.ctr + CTR_DECIDED, ws.ctr + CTR_AUX);
   if (undecided > 32) {
     k_res_block<<<static_cast<unsigned>(std::min<uint64_t>(148 * 6, undecided / 33 + 1)), RB_T, 0, s>>>(rc, pieces, static_cast<uint32_t>(each), count, start, place, members, g.fh, g.fc, und, scc_id,
                                                                                                        ws.ctr + CTR_DECIDED, ws.ctr + CTR_AUX);
