@@ -740,7 +740,7 @@ bt_solve(bt_args const& a, uint32_t gi, bt_group const& g, rs_piece& piece)
 // access instead of a trip to L2, and a level needs one block barrier (its
 // append counter rotates over three slots, so no thread waits for a reset).
 // What then bounds it is DRAM: a few hundred graphs in flight overflow L2,
-// and a row read at random costs 64 bytes per access.  So the wide passes
+// and a row read at random costs a 128-byte line per access.  So the wide passes
 // (bottom-up levels, the recount after an SCC) go through the vertices in id
 // order, 32 lanes on neighbouring vertices; live degrees take one byte per
 // direction (graphs with a row of BB_DEG8 or more entries: 32 bits); and

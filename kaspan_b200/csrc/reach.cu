@@ -1883,7 +1883,11 @@ run_joint(fwbw_args const& a, fwbw_smem& sm, uint32_t pivot, uint32_t n_und, uin
         // several start vertices where the searches grow slowly and most of the
         // graph is undecided (near the giant-component threshold of a random
         // graph, mean degree below 1.7, less than 2/3 are and most candidates
-        // lie outside the SCC: a restart for nothing), and no row is on a cut
+        // lie outside the SCC: a restart for nothing; G(n, m) n 300,000 and 3 M
+        // without this limit, undecided 0.57: 389 -> 478 and 1,040 -> 1,157 us,
+        // 0.60: 354 -> 443 and 954 -> 1,059, 0.64 the same.  Above it the starts
+        // cost those graphs 1 to 3%, and near-critical geometric ones up to 6%,
+        // where geometric graphs of mean degree 8 gain 1.7 to 4.3 times), and no row is on a cut
         // list: its vertex, and what only it leads to, may belong to the SCC
         // and be in neither set yet, and a restart would keep them out of C
         // for good; block-uniform (no sweep runs since the last barrier)
@@ -3064,7 +3068,12 @@ launch_persistent(kspn_context* ctx, dgraph const& g, uint32_t* und, uint32_t* s
   void* args[]    = { &a };
   barrier_for_grid(ctx, fwbw_grid(ctx, g));
   // the opening saves at most three levels (27 us) where the mean degree is 8
-  // and more; on such a graph of THIN_MAX vertices and edges its spills cost as much
+  // and more; on such a graph of THIN_MAX vertices and edges its spills cost as
+  // much.  Whole call with / without it: G(n, m) n 5 M, degree 8.5 (48 M): 657 /
+  // 669 us; n 20 M (190 M): 1,612 / 1,618; R-MAT degree 16, scale 22 and 24
+  // (280 M): 240 / 240, 451 / 449; G(n, m) n 30 M, degree 16 (510 M): 2,048 /
+  // 2,045; R-MAT scale 25 and 26 (1,130 M): 734 / 729, 1,213 / 1,200.  (R-MAT
+  // of degree 9, scale 22 and 24, loses below the line too: 251 / 243, 448 / 438.)
   bool const  thin   = !a.model && (g.m < 8ull * g.n || g.n + g.m < THIN_MAX);
   auto* const kernel = thin ? reinterpret_cast<void const*>(&k_fwbw<4, true>) : reinterpret_cast<void const*>(&k_fwbw<4, false>);
   KSPN_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(fwbw_grid(ctx, g)), dim3(R_THREADS), args, 0, ctx->stream));
