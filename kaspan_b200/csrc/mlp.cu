@@ -99,10 +99,10 @@ k_mlp_forward(uint32_t count, float const* __restrict__ feat, float const* __res
 // memory once.
 // Bound: issue slots (~100 FMAs and ~60 other instructions per sample and
 // lane).  65,536 samples: 391 us with the weights in shared memory (row
-// `lane` of W2: all lanes on one bank) and a shuffle per hidden unit.  Longer
-// sums per lane before the atomic additions make it the more exact one too
-// (gradient against 64 bits, 1,000 to 200,000 samples: median error 0.4 to
-// 1.9e-07 of the largest entry, 1.4 to 7.3e-07 before).
+// `lane` of W2: all lanes on one bank) and a shuffle per hidden unit.  Gradient
+// against 64 bits (1,000 to 200,000 samples, repeated runs: the atomic
+// additions' order varies): median error 0.4 to 1.9e-07 of the largest entry,
+// 1.4 to 7.3e-07 before.
 constexpr int MG_WARPS = 12; // 384 threads of up to 168 registers: one block per SM
 
 __global__ void __launch_bounds__(MG_WARPS * 32, 1)
