@@ -13,6 +13,7 @@ import pytest
 import kaspan_b200 as K
 import kaspan_b200.graphs as KG
 import oracle as O
+from test_gpu_seeded_search import build
 
 pytestmark = pytest.mark.gpu
 
@@ -64,3 +65,39 @@ def test_hub_on_the_cut_list(ctx, beyond, mirror, validate):
         got = st.as_dict()
         assert got["pivot"] == pivot
         assert got["heavy"]["cut_rows"] > 0 and got["search_worklist"] == 1
+
+
+@pytest.mark.parametrize("mirror", [False, True])
+@pytest.mark.parametrize("kind", ["upstream", "both", "through"])
+def test_rows_cut_after_the_restart(ctx, kind, mirror):
+    """Thin from the first level on, so no sweep comes before the start
+    vertices; some of them outside the component, so that both sets restart
+    and sweep; hubs on the component's cycle behind 3000 sources each, whose
+    rows those sweeps cut."""
+    import torch
+
+    n0, s, d = build(kind)
+    first, hubs = 3 * HUB, (23000, 61000, 90500)  # the sources' ids come first in the hubs' rows
+    pivot = first + np.bincount(s, minlength=n0).argmax()
+    rng = np.random.default_rng(5)
+    main = np.flatnonzero(np.bincount(s, minlength=n0) == 1) + first
+    e = [(s.astype(np.int64) + first, d.astype(np.int64) + first)]
+    for i, h in enumerate(hubs):
+        e.append((np.arange(i * HUB, (i + 1) * HUB), np.full(HUB, main[np.searchsorted(main, h)])))
+    fan = rng.choice(main[1000:2000], 100, replace=False)  # more in * out than a hub's 3001 x 1
+    e += [(np.full(100, pivot), fan), (fan, np.full(100, pivot))]
+    s, d = (np.concatenate([x[i] for x in e]).astype(np.uint32) for i in (0, 1))
+    if mirror:
+        s, d = d, s
+    n = n0 + first
+    G = KG.from_edges(ctx, n, *(torch.from_numpy(x.view(np.int32)).cuda() for x in (s, d)))
+    fwh, fwc, bwh, bwc = G.to_host()
+    want = O.tarjan(O.Graph(n, fwh, fwc, bwh, bwc))
+    out = torch.empty(n, dtype=torch.int32, device="cuda")
+    for after in (0, 1):
+        st = K.Stats()
+        ctx.scc_device(n, G.m, G.fwh, G.fwc, G.bwh, G.bwc, out, K.default_options(aw_exact_after=after), st)
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), want)
+        got = st.as_dict()
+        assert got["pivot"] == pivot and got["search_worklist"] == 1
+        assert got["levels_bottom_up"] > 0 and got["heavy"]["cut_rows"] == len(hubs) and got["heavy"]["fixups"] > 0
